@@ -320,17 +320,19 @@ __device__ __forceinline__ void store_images_3d(double* __restrict__ q, int64_t 
 // carries no run-time EOS branch.
 // Occupancy: the tiles' phases wait at barriers and on dependency chains, and
 // more resident CTAs fill those waits.  Where the shared memory of a launch
-// leaves room for them (no passive scalars), the 2-D FP64 tile runs three CTAs
-// per SM (80 registers, some spilled; KH 2048^2: 1.19 -> 1.02 ms per step;
-// 16x8 tiles at five CTAs per SM: 1.15 ms).  The other tiles (0 here) keep
-// the compiler's register choice, which already gives the FP32-mixed 2-D
-// 256-thread tiles three CTAs per SM and the 3-D tile two (asking for a
-// minimum of one block instead lets it take more registers: RT 256^2 x 512
-// with a passive scalar 8.8 -> 14.3 ms).
+// leaves room for them the 2-D FP64 tile runs two CTAs per SM (128 registers,
+// some spilled; KH 2048^2 with a passive scalar 1.75 ms per step unbounded,
+// 1.10 ms so).  The straight-line quotients hold more values at once than the
+// branching divisions did: three CTAs (80 registers) spill 1.5 KB per thread.
+// The other tiles (0 here) keep the compiler's register choice: the 3-D FP64
+// tile at one CTA and 255 registers measures as at two and 128 (a spherical
+// 96 x 64 x 50 step 0.22 ms), and asking for a minimum of one block lets the
+// FP32-mixed 3-D tile take too many registers (RT 256^2 x 512 with a passive
+// scalar 8.8 -> 14.3 ms).
 template <int ND, bool EXACT, int TX, int TY, int TZ>
 constexpr int fused_min_blocks()
 {
-    return (EXACT && ND == 2) ? 3 : 0;
+    return (EXACT && ND == 2) ? 2 : 0;
 }
 
 // tma (2-D and 3-D): the FP64 tile plus its halo arrives as one tensor box
@@ -416,7 +418,7 @@ __device__ __forceinline__ void fused_step_body(const GridDev& g, const StateDev
         nvalid[d] = d < ND ? min(tdim, g.nx[d] - t0[d]) : 1;
     }
 
-    const exact::Eos eeos{g.gamma, g.gamma_m1, g.mmw, EOSK};
+    const exact::Eos eeos = exact::make_eos(g.gamma, g.gamma_m1, g.mmw, EOSK);
     const fast::Eos feos{(float)g.gamma, (float)g.gamma_m1, (float)(1.0 / g.gamma_m1)};
 
     // ---- phase 1: state tile + halo -> primitives --------------------------
@@ -569,29 +571,23 @@ __device__ __forceinline__ void fused_step_body(const GridDev& g, const StateDev
                 dl_m = g.dx[idim][gcc[idim] - 1];
                 dl_p = g.dx[idim][gcc[idim] + 1];
             }
+            if constexpr (EXACT) {
+                double vm[NV], vc[NV], vp[NV];
+#pragma unroll
+                for (int v = 0; v < NV; ++v) {
+                    vm[v] = sp[v * S::NP + lc - lstride[idim]];
+                    vc[v] = sp[v * S::NP + lc];
+                    vp[v] = sp[v * S::NP + lc + lstride[idim]];
+                }
+                exact::faces<NV>(EOSK, g.limiter, g.uniform_cart, vm, vc, vp, dl_m, dl, dl_p, fp[0][idim], fp[1][idim]);
+                continue;
+            }
 #pragma unroll
             for (int v = 0; v < NV; ++v) {
                 const R vc = sp[v * S::NP + lc];
                 const R vp = sp[v * S::NP + lc + lstride[idim]];
                 const R vm = sp[v * S::NP + lc - lstride[idim]];
-                if constexpr (EXACT && EOSK == EOS_PERFECT_GAS_FAST) {
-                    // fast FP64 on a uniform grid: the limiter of the raw
-                    // differences, halved (positive homogeneity, as below)
-                    if (g.uniform_cart) {
-                        const double sh = 0.5 * exact::slope(g.limiter, vp - vc, vc - vm, EOSK);
-                        fp[0][idim][v] = vc - sh;
-                        fp[1][idim][v] = vc + sh;
-                    } else {
-                        const double slope =
-                            exact::slope(g.limiter, (vp - vc) / ((dl + dl_p) / 2), (vc - vm) / ((dl_m + dl) / 2), EOSK);
-                        fp[0][idim][v] = vc - ((dl / 2) * slope);
-                        fp[1][idim][v] = vc + ((dl / 2) * slope);
-                    }
-                } else if constexpr (EXACT) {
-                    const double slope = exact::slope(g.limiter, (vp - vc) / ((dl + dl_p) / 2), (vc - vm) / ((dl_m + dl) / 2));
-                    fp[0][idim][v] = vc - ((dl / 2) * slope);
-                    fp[1][idim][v] = vc + ((dl / 2) * slope);
-                } else if (g.uniform_cart) {
+                if (g.uniform_cart) {
                     // dl/2 * limiter(dR/dl, dL/dl) = limiter(dR, dL)/2 (every limiter
                     // is positively homogeneous of degree 1)
                     const float s = 0.5f * fast::limited(g.limiter, vp - vc, vc - vm);
@@ -607,14 +603,16 @@ __device__ __forceinline__ void fused_step_body(const GridDev& g, const StateDev
                 }
             }
         }
-        // face conservatives (hydro_reconstruction.hpp:111-126)
+        // face conservatives (hydro_reconstruction.hpp:111-126); in FP64 the
+        // fluxes of the predictor with them (they share rho u and E)
         R fc[2][ND][NV];
+        R ff[EXACT ? 2 : 1][EXACT ? ND : 1][EXACT ? NV : 1];
 #pragma unroll
         for (int idim = 0; idim < ND; ++idim) {
 #pragma unroll
             for (int s = 0; s < 2; ++s) {
                 if constexpr (EXACT) {
-                    exact::to_cons<ND>(eeos, fp[s][idim], fc[s][idim]);
+                    exact::to_cons_flux<ND>(eeos, fp[s][idim], idim, fc[s][idim], ff[s][idim]);
                 } else {
                     fast::to_cons<ND>(feos, fp[s][idim], fc[s][idim]);
                 }
@@ -654,10 +652,9 @@ __device__ __forceinline__ void fused_step_body(const GridDev& g, const StateDev
         R mflux[2][ND]; // mass fluxes of the face states before the update (passive scalars)
 #pragma unroll
         for (int idim = 0; idim < ND; ++idim) {
-            R fL[NV], fR[NV];
             if constexpr (EXACT) {
-                exact::flux_prim<ND>(eeos, fp[0][idim], idim, fL);
-                exact::flux_prim<ND>(eeos, fp[1][idim], idim, fR);
+                const R* fL = ff[0][idim];
+                const R* fR = ff[1][idim];
                 mflux[0][idim] = fL[0];
                 mflux[1][idim] = fR[0];
                 const double dtodv = dth / dv_c;
@@ -716,6 +713,7 @@ __device__ __forceinline__ void fused_step_body(const GridDev& g, const StateDev
                     }
                 }
             } else {
+                R fL[NV], fR[NV];
                 fast::flux_prim<ND>(feos, fp[0][idim], idim, fL);
                 fast::flux_prim<ND>(feos, fp[1][idim], idim, fR);
                 mflux[0][idim] = fL[0];
@@ -800,10 +798,7 @@ __device__ __forceinline__ void fused_step_body(const GridDev& g, const StateDev
                     const double dl = g.dx[idim][gcc[idim]];
                     const double dl_m = g.dx[idim][gcc[idim] - 1];
                     const double dl_p = g.dx[idim][gcc[idim] + 1];
-                    const double slope = exact::slope(g.limiter, (vp - vc) / ((dl + dl_p) / 2), (vc - vm) / ((dl_m + dl) / 2),
-                                                      EOSK);
-                    xf[0][idim] = vc - ((dl / 2) * slope);
-                    xf[1][idim] = vc + ((dl / 2) * slope);
+                    exact::faces<1>(EOSK, g.limiter, false, &vm, &vc, &vp, dl_m, dl, dl_p, &xf[0][idim], &xf[1][idim]);
                 } else if (g.uniform_cart) {
                     const float sl = 0.5f * fast::limited(g.limiter, vp - vc, vc - vm);
                     xf[0][idim] = vc - sl;
@@ -1192,14 +1187,7 @@ __device__ __forceinline__ void fused_step_body(const GridDev& g, const StateDev
         // health check (main.cpp:397-425) and CFL of the new state (time_step.hpp:55-77)
         double evol, inv_rho_u[ND], sound;
         if constexpr (EXACT) {
-            evol = qn[1 + ND] - exact::ek_cons<ND>(qn);
-            double pr[NV];
-            exact::to_prim<ND>(eeos, qn, pr);
-            sound = exact::sound(eeos, pr[0], pr[1 + ND]);
-#pragma unroll
-            for (int d = 0; d < ND; ++d) {
-                inv_rho_u[d] = fabs(pr[1 + d]);
-            }
+            exact::state_speeds<ND>(eeos, qn, evol, sound, inv_rho_u);
         } else {
             double r = (double)__frcp_rn((float)qn[0]);
             r = r * (2.0 - qn[0] * r);

@@ -3,8 +3,9 @@
 // Each function keeps the association order of the reference expression it
 // restates, and the translation units that include this header are built
 // with --fmad=false, so the device results round exactly like the reference's
-// FP64 CPU build (IEEE division and square root are the CUDA defaults for
-// double).  State vectors are [rho, v_0..v_{ND-1}, E or P].
+// FP64 CPU build: every quotient and square root is the rounded one, formed
+// from shared reciprocals (quot64.cuh) or, out of their range, by IEEE
+// division and square root.  State vectors are [rho, v_0..v_{ND-1}, E or P].
 //
 // Eos kind EOS_PERFECT_GAS_FAST selects the fast-FP64 forms instead (used by
 // the fused kernels of the fast-FP64 precision, built with FMA contraction):
@@ -17,17 +18,29 @@
 #pragma once
 
 #include "hcl_device.cuh"
+#include "quot64.cuh"
 
 namespace hcl::exact {
 
 struct Eos {
     double gamma, gamma_m1, mmw;
-    int kind; // EOS_PERFECT_GAS or EOS_RAD_GAS
+    int kind; // EOS_PERFECT_GAS, EOS_RAD_GAS or EOS_PERFECT_GAS_FAST
+    // the perfect gas's constant denominators (perfect_gas.hpp:46-83): mu m_p
+    // and mu m_p (gamma - 1); consts_ok: both usable as such
+    q64::Den mk, ev;
+    bool consts_ok;
 };
+
+__device__ __forceinline__ Eos make_eos(double gamma, double gamma_m1, double mmw, int kind)
+{
+    const double b = mmw * kMp;
+    const double c = mmw * kMp * gamma_m1;
+    return Eos{gamma, gamma_m1, mmw, kind, q64::Den{b, 1.0 / b}, q64::Den{c, 1.0 / c}, q64::den_ok(b) && q64::den_ok(c)};
+}
 
 __device__ __forceinline__ Eos eos_of(const GridDev& g)
 {
-    return Eos{g.gamma, g.gamma_m1, g.mmw, g.eos};
+    return make_eos(g.gamma, g.gamma_m1, g.mmw, g.eos);
 }
 
 // thermodynamics/rad_gas.hpp:47-146: gas plus radiation.  The temperature
@@ -140,7 +153,7 @@ __device__ __forceinline__ double pres_from_evol(const Eos& e, double rho, doubl
     }
     return pres_from_temp(e, rho, temp_from_evol(e, rho, evol));
 }
-__device__ __forceinline__ double sound(const Eos& e, double rho, double P)
+__device__ __forceinline__ double plain_sound(const Eos& e, double rho, double P)
 {
     if (e.kind == EOS_RAD_GAS) {
         return rad::sound(e, rho, P);
@@ -148,6 +161,10 @@ __device__ __forceinline__ double sound(const Eos& e, double rho, double P)
     return sqrt(e.gamma * P / rho);
 }
 
+// The step's algebra with the plain operators: what every fast form below
+// falls back to when an operand is near overflow or underflow, the RadGas
+// path, and the low-Mach solver's own expressions.
+namespace plain {
 // hydro/euler_equations.hpp:41-59
 template <int ND>
 __device__ __forceinline__ double ek_cons(const double* c)
@@ -271,12 +288,12 @@ template <int ND>
 __device__ __forceinline__ void riemann(const Eos& e, int solver, const double* cL, const double* cR, int l, double* f)
 {
     double pL[ND + 2], pR[ND + 2];
-    to_prim<ND>(e, cL, pL);
-    to_prim<ND>(e, cR, pR);
+    plain::to_prim<ND>(e, cL, pL);
+    plain::to_prim<ND>(e, cR, pR);
     const double PL = pL[1 + ND];
     const double PR = pR[1 + ND];
-    const double aL = sound(e, pL[0], PL);
-    const double aR = sound(e, pR[0], PR);
+    const double aL = plain_sound(e, pL[0], PL);
+    const double aR = plain_sound(e, pR[0], PR);
     const double uL = pL[1 + l];
     const double uR = pR[1 + l];
     if (solver == RS_SPLITTING) {
@@ -299,8 +316,8 @@ __device__ __forceinline__ void riemann(const Eos& e, int solver, const double* 
     const double wsL = fmin(uL - aL, uR - aR);
     const double wsR = fmax(uL + aL, uR + aR);
     double fL[ND + 2], fR[ND + 2];
-    flux_prim<ND>(e, pL, l, fL);
-    flux_prim<ND>(e, pR, l, fR);
+    plain::flux_prim<ND>(e, pL, l, fL);
+    plain::flux_prim<ND>(e, pR, l, fR);
     if (solver == RS_HLL) {
         // :31-58
         const double neg_wsL = fmin(wsL, 0.);
@@ -353,6 +370,547 @@ __device__ __forceinline__ void riemann(const Eos& e, int solver, const double* 
     f[1 + l] = (rho_star * ustar * ustar) + pstar;
     const double E_star = ((S - un) / (S - ustar) * cs[1 + ND]) + ((ustar - un) / (S - ustar) * ((ustar * cs[0] * (S - un)) + ps[1 + ND]));
     f[1 + ND] = flux_hllc(fs[1 + ND], cs[1 + ND], E_star, S);
+}
+} // namespace plain
+
+// hydro/euler_equations.hpp:41-59
+using plain::ek_cons;
+using plain::ek_prim;
+
+// ---- the same results with shared reciprocals (quot64.cuh) ------------------
+// Each *_core evaluates a group of expressions straight through and gathers
+// its operands in two ranges: S, and Z for numerators that may be zero.  Where
+// both hold every quotient and root is the rounded one.  Otherwise the caller
+// looks at the Z operands one by one and, unless those outside are all zeros,
+// redoes the group with plain operators, out of line.  Scalings by powers of two (the /2 of the kinetic energy, the 4/2
+// and 2/2 of the limiters) are folded, which is exact in that range.
+template <int ND>
+static __device__ __noinline__ void to_prim_slow(Eos e, const double* c, double* p)
+{
+    plain::to_prim<ND>(e, c, p);
+}
+template <int ND>
+static __device__ __noinline__ void to_cons_flux_slow(Eos e, const double* p, int l, double* c, double* f)
+{
+    plain::to_cons<ND>(e, p, c);
+    plain::flux_prim<ND>(e, p, l, f);
+}
+template <int ND>
+static __device__ __noinline__ void riemann_slow(Eos e, int solver, const double* cL, const double* cR, int l, double* f)
+{
+    plain::riemann<ND>(e, solver, cL, cR, l, f);
+}
+static __device__ __noinline__ double sound_slow(Eos e, double rho, double P)
+{
+    return plain_sound(e, rho, P);
+}
+
+// hydro/euler_equations.hpp:111-122.  r, k: the denominators rho and rho kb;
+// evol: the internal energy.  S holds rho and P, Z the momenta.
+template <int ND>
+__device__ __forceinline__ void prim_core(const Eos& e, const double* c, double* p, q64::Den& r, q64::Den& k,
+                                          double& evol, q64::Range& S, q64::Range& Z)
+{
+    r = q64::den(c[0]);
+    p[0] = c[0];
+    if (e.kind == EOS_PERFECT_GAS_FAST) {
+        double mu = 0;
+#pragma unroll
+        for (int d = 0; d < ND; ++d) {
+            p[1 + d] = c[1 + d] * r.y;
+            mu += c[1 + d] * p[1 + d];
+        }
+        evol = c[1 + ND] - 0.5 * mu;
+        p[1 + ND] = e.gamma_m1 * evol;
+        S.add(c[0], p[1 + ND]);
+        return;
+    }
+    double norm = 0;
+#pragma unroll
+    for (int d = 0; d < ND; ++d) {
+        norm += c[1 + d] * c[1 + d];
+        p[1 + d] = q64::quo(c[1 + d], r);
+    }
+    evol = __fma_rn(-0.5, q64::quo(norm, r), c[1 + ND]);
+    const double kb = c[0] * kKb;
+    k = q64::den_from(kb, r.y * (1 / kKb));
+    p[1 + ND] = q64::quo(kb * q64::quo(evol * e.mmw * kMp * e.gamma_m1, k), e.mk);
+    S.add(c[0], p[1 + ND]);
+    S.low(c[0]);
+    S.low(kb);
+    Z.add(c[1], ND >= 2 ? c[2] : c[1]);
+    if constexpr (ND == 3) {
+        Z.add(c[3]);
+    }
+}
+// the Z operands of prim_core
+template <int ND>
+__device__ __forceinline__ bool prim_zeros(const Eos& e, const double* c)
+{
+    bool ok = true;
+    if (e.kind != EOS_PERFECT_GAS_FAST) {
+#pragma unroll
+        for (int d = 0; d < ND; ++d) {
+            ok = ok && q64::within0(c[1 + d]);
+        }
+    }
+    return ok;
+}
+
+template <int ND>
+__device__ __forceinline__ void to_prim(const Eos& e, const double* c, double* p)
+{
+    if (e.kind == EOS_RAD_GAS) {
+        plain::to_prim<ND>(e, c, p);
+        return;
+    }
+    q64::Den r, k;
+    double evol;
+    q64::Range S(e.consts_ok), Z;
+    prim_core<ND>(e, c, p, r, k, evol, S, Z);
+    if (!(S.ok() && Z.ok())) {
+        if (!(S.ok() && prim_zeros<ND>(e, c))) {
+            double ct[ND + 2], pt[ND + 2];
+#pragma unroll
+            for (int v = 0; v < ND + 2; ++v) {
+                ct[v] = c[v];
+            }
+            to_prim_slow<ND>(e, ct, pt);
+#pragma unroll
+            for (int v = 0; v < ND + 2; ++v) {
+                p[v] = pt[v];
+            }
+        }
+    }
+}
+
+// e(rho, P) of the perfect gas through the temperature; k: the denominator
+// rho kb (perfect_gas.hpp:46-83).  In range where rho and P are.
+__device__ __forceinline__ double evol_core(const Eos& e, double P, const q64::Den& k)
+{
+    return q64::quo(k.b * q64::quo(P * e.mmw * kMp, k), e.ev);
+}
+
+// hydro/euler_equations.hpp:124-134 and :72-86: the conservative state of a
+// face and its flux along l, which share rho u_l and E
+template <int ND>
+__device__ __forceinline__ void cons_flux_core(const Eos& e, const double* p, int l, double* c, double* f, q64::Range& S)
+{
+    double evol;
+    if (e.kind == EOS_PERFECT_GAS_FAST) {
+        evol = p[1 + ND] * (1.0 / e.gamma_m1);
+    } else {
+        const double kb = p[0] * kKb;
+        S.add(p[0], p[1 + ND]);
+        S.low(kb);
+        evol = evol_core(e, p[1 + ND], q64::den(kb));
+    }
+    double norm = 0;
+    c[0] = p[0];
+#pragma unroll
+    for (int d = 0; d < ND; ++d) {
+        c[1 + d] = p[0] * p[1 + d];
+        norm += p[1 + d] * p[1 + d];
+    }
+    c[1 + ND] = __fma_rn(0.5, p[0] * norm, evol);
+    f[0] = c[1 + l];
+#pragma unroll
+    for (int d = 0; d < ND; ++d) {
+        f[1 + d] = c[1 + l] * p[1 + d];
+    }
+    f[1 + l] += p[1 + ND];
+    f[1 + ND] = p[1 + l] * (c[1 + ND] + p[1 + ND]);
+}
+
+template <int ND>
+__device__ __forceinline__ void to_cons_flux(const Eos& e, const double* p, int l, double* c, double* f)
+{
+    if (e.kind == EOS_RAD_GAS) {
+        plain::to_cons<ND>(e, p, c);
+        plain::flux_prim<ND>(e, p, l, f);
+        return;
+    }
+    q64::Range S(e.consts_ok);
+    cons_flux_core<ND>(e, p, l, c, f, S);
+    if (!S.ok()) {
+        double pt[ND + 2], ct[ND + 2], ft[ND + 2];
+#pragma unroll
+        for (int v = 0; v < ND + 2; ++v) {
+            pt[v] = p[v];
+        }
+        to_cons_flux_slow<ND>(e, pt, l, ct, ft);
+#pragma unroll
+        for (int v = 0; v < ND + 2; ++v) {
+            c[v] = ct[v];
+            f[v] = ft[v];
+        }
+    }
+}
+template <int ND>
+__device__ __forceinline__ void to_cons(const Eos& e, const double* p, double* c)
+{
+    double f[ND + 2];
+    to_cons_flux<ND>(e, p, 0, c, f);
+}
+template <int ND>
+__device__ __forceinline__ void flux_prim(const Eos& e, const double* p, int l, double* f)
+{
+    double c[ND + 2];
+    to_cons_flux<ND>(e, p, l, c, f);
+}
+
+__device__ __forceinline__ double sound(const Eos& e, double rho, double P)
+{
+    if (e.kind == EOS_RAD_GAS) {
+        return plain_sound(e, rho, P);
+    }
+    if (!(q64::den_ok(rho) && q64::within(P))) {
+        return sound_slow(e, rho, P);
+    }
+    return q64::root(q64::quo(e.gamma * P, q64::den(rho)));
+}
+
+// What the health check and the CFL need of a new state: the internal energy
+// (main.cpp:397-425), |u_d| and the sound speed (time_step.hpp:55-77).
+template <int ND>
+static __device__ __noinline__ void state_speeds_slow(Eos e, const double* q, double* out)
+{
+    double pr[ND + 2];
+    out[0] = q[1 + ND] - plain::ek_cons<ND>(q);
+    plain::to_prim<ND>(e, q, pr);
+    out[1] = plain_sound(e, pr[0], pr[1 + ND]);
+    for (int d = 0; d < ND; ++d) {
+        out[2 + d] = fabs(pr[1 + d]);
+    }
+}
+template <int ND>
+__device__ __forceinline__ void state_speeds(const Eos& e, const double* q, double& evol, double& snd, double* absu)
+{
+    bool slow = e.kind == EOS_RAD_GAS;
+    if (e.kind != EOS_RAD_GAS) {
+        double pr[ND + 2];
+        q64::Den r, k;
+        q64::Range S(e.consts_ok), Z;
+        prim_core<ND>(e, q, pr, r, k, evol, S, Z);
+        snd = q64::root(q64::quo(e.gamma * pr[1 + ND], r));
+#pragma unroll
+        for (int d = 0; d < ND; ++d) {
+            absu[d] = fabs(pr[1 + d]);
+        }
+        if (!(S.ok() && Z.ok())) {
+            slow = !(S.ok() && prim_zeros<ND>(e, q));
+        }
+    }
+    if (slow) {
+        double qt[ND + 2], ot[ND + 2];
+#pragma unroll
+        for (int v = 0; v < ND + 2; ++v) {
+            qt[v] = q[v];
+        }
+        state_speeds_slow<ND>(e, qt, ot);
+        evol = ot[0];
+        snd = ot[1];
+#pragma unroll
+        for (int d = 0; d < ND; ++d) {
+            absu[d] = ot[2 + d];
+        }
+    }
+}
+
+// hydro/slope_limiters.hpp:18-87 on the two one-sided quotients: limited_core
+// returns the slope, halved for van Leer (4 ratio / 2 folded), so that a face
+// lies limited_core * limited_width from the centre.  FAST: the raw-difference
+// forms.
+template <int LIM>
+__device__ __forceinline__ double limited_width(double dl)
+{
+    return LIM == LIM_VANLEER ? dl : dl / 2;
+}
+// Z holds the quotients and the limiter's own denominator: in range wherever
+// both quotients are normal-sized, so what is left to the one-by-one look
+// (limited_ok) is flat or extreme data.
+template <int LIM>
+__device__ __forceinline__ double limited_den(double ratio)
+{
+    return LIM == LIM_VANLEER ? (ratio + 1) * (ratio + 1) : (LIM == LIM_MINMOD ? 1 + ratio : (ratio * ratio) + 1);
+}
+template <int LIM>
+__device__ __forceinline__ double limited_core(double dR, double dL, q64::Range& Z)
+{
+    const double ratio = q64::quo(dR, q64::den(dL));
+    const double b = limited_den<LIM>(ratio);
+    const double num = LIM == LIM_MINMOD ? fmin(1., ratio) : (dR + dL) * ratio;
+    double s = q64::quo(num, q64::den(b));
+    if constexpr (LIM == LIM_MINMOD) {
+        s = s * (dL + dR);
+    }
+    Z.add(dR, dL);
+    Z.add(b);
+    Z.low(dL);
+    Z.low(b);
+    return dL * dR > 0 ? s : 0.0;
+}
+template <int LIM>
+__device__ __forceinline__ bool limited_ok(double dR, double dL)
+{
+    return !(dL * dR > 0) ||
+           (q64::den_ok(dL) && q64::within(dR) && q64::den_ok(limited_den<LIM>(q64::quo(dR, q64::den(dL)))));
+}
+// the raw-difference forms of the fast kind
+template <int LIM>
+__device__ __forceinline__ double limited_fast(double dR, double dL, q64::Range& Z)
+{
+    const double prod = dR * dL;
+    double s;
+    if constexpr (LIM == LIM_MINMOD) {
+        s = fabs(dR) < fabs(dL) ? dR : dL;
+    } else {
+        const double num = LIM == LIM_VANLEER ? prod : prod * (dR + dL);
+        const double b = LIM == LIM_VANLEER ? dR + dL : dR * dR + dL * dL;
+        s = q64::quo(num, q64::den(b));
+        Z.add(b);
+    }
+    return prod > 0 ? s : 0.0;
+}
+template <int LIM>
+__device__ __forceinline__ bool limited_fast_ok(double dR, double dL)
+{
+    return LIM == LIM_MINMOD || !(dR * dL > 0) ||
+           (q64::within(dR) && q64::within(dL) && q64::within(LIM == LIM_VANLEER ? dR + dL : dR * dR + dL * dL));
+}
+
+// limited_linear_reconstruction.hpp:46-64 for NV variables of one cell along
+// one dimension: values m, c, p of the cell and its neighbours, the distances
+// hL, hR to them and half the cell's width (raw differences of the fast kind:
+// 1, 1 and 1/2).
+template <int NV>
+static __device__ __noinline__ void faces_slow(int kind, int lim, const double* m, const double* c, const double* p,
+                                               double hL, double hR, double half, double* lo, double* hi)
+{
+    for (int v = 0; v < NV; ++v) {
+        const double s = half * plain::slope(lim, (p[v] - c[v]) / hR, (c[v] - m[v]) / hL, kind);
+        lo[v] = c[v] - s;
+        hi[v] = c[v] + s;
+    }
+}
+// ld(k, v): variable v of the cell (k = 1) and its neighbours (0, 2);
+// ld_again(k, v) the same for the rare second look, so that a caller with the
+// values in memory need not keep them in registers.
+template <int NV, int LIM, class Ld, class LdAgain>
+__device__ __forceinline__ void faces_ld(int kind, const Ld& ld, const LdAgain& ld_again, const q64::Den& hL,
+                                         const q64::Den& hR, double half, double* lo, double* hi)
+{
+    const bool fast = kind == EOS_PERFECT_GAS_FAST;
+    const double w = LIM == LIM_VANLEER ? 2 * half : half;
+    q64::Range Z;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+        const double c = ld(1, v);
+        const double R = fast ? (ld(2, v) - c) * hR.y : q64::quo(ld(2, v) - c, hR);
+        const double L = fast ? (c - ld(0, v)) * hL.y : q64::quo(c - ld(0, v), hL);
+        const double s = w * (fast ? limited_fast<LIM>(R, L, Z) : limited_core<LIM>(R, L, Z));
+        lo[v] = c - s;
+        hi[v] = c + s;
+    }
+    const bool h_ok = q64::den_ok(hR.b) && q64::den_ok(hL.b);
+    if (!(h_ok && Z.ok())) {
+        double mt[NV], ct[NV], pt[NV];
+        bool ok = h_ok;
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            mt[v] = ld_again(0, v);
+            ct[v] = ld_again(1, v);
+            pt[v] = ld_again(2, v);
+            const double aR = pt[v] - ct[v], aL = ct[v] - mt[v];
+            ok = ok && (fast ? limited_fast_ok<LIM>(aR * hR.y, aL * hL.y)
+                             : (q64::within0(aR) && q64::within0(aL) &&
+                                limited_ok<LIM>(q64::quo(aR, hR), q64::quo(aL, hL))));
+        }
+        if (!ok) {
+            double lt[NV], ht[NV];
+            faces_slow<NV>(kind, LIM, mt, ct, pt, hL.b, hR.b, half, lt, ht);
+#pragma unroll
+            for (int v = 0; v < NV; ++v) {
+                lo[v] = lt[v];
+                hi[v] = ht[v];
+            }
+        }
+    }
+}
+template <int NV, int LIM>
+__device__ __forceinline__ void faces_den(int kind, const double* m, const double* c, const double* p, const q64::Den& hL,
+                                          const q64::Den& hR, double half, double* lo, double* hi)
+{
+    const auto ld = [&](int k, int v) { return k == 0 ? m[v] : (k == 1 ? c[v] : p[v]); };
+    faces_ld<NV, LIM>(kind, ld, ld, hL, hR, half, lo, hi);
+}
+template <int NV, int LIM>
+__device__ __forceinline__ void faces_lim(int kind, bool uniform, const double* m, const double* c, const double* p,
+                                          double dl_m, double dl, double dl_p, double* lo, double* hi)
+{
+    if (kind == EOS_PERFECT_GAS_FAST && uniform) {
+        faces_den<NV, LIM>(kind, m, c, p, q64::Den{1.0, 1.0}, q64::Den{1.0, 1.0}, 0.5, lo, hi);
+    } else {
+        faces_den<NV, LIM>(kind, m, c, p, q64::den((dl_m + dl) / 2), q64::den((dl + dl_p) / 2), dl / 2, lo, hi);
+    }
+}
+template <int NV>
+__device__ __forceinline__ void faces(int kind, int lim, bool uniform, const double* m, const double* c, const double* p,
+                                      double dl_m, double dl, double dl_p, double* lo, double* hi)
+{
+    if (lim == LIM_VANLEER) {
+        faces_lim<NV, LIM_VANLEER>(kind, uniform, m, c, p, dl_m, dl, dl_p, lo, hi);
+    } else if (lim == LIM_MINMOD) {
+        faces_lim<NV, LIM_MINMOD>(kind, uniform, m, c, p, dl_m, dl, dl_p, lo, hi);
+    } else if (lim == LIM_VANALBADA) {
+        faces_lim<NV, LIM_VANALBADA>(kind, uniform, m, c, p, dl_m, dl, dl_p, lo, hi);
+    } else {
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            lo[v] = c[v] - ((dl / 2) * 0.0);
+            hi[v] = c[v] + ((dl / 2) * 0.0);
+        }
+    }
+}
+
+// hydro/riemann_solver.hpp:22-134 (HLL and HLLC).  HLLC needs the flux of the
+// side the star state lies on only.  zeros: the operands besides the momenta
+// that may be zero and are.
+template <int ND, int RS>
+__device__ __forceinline__ void riemann_core(const Eos& e, const double* cL, const double* cR, int l, double* f,
+                                             q64::Range& S, q64::Range& Z, bool& zeros)
+{
+    constexpr int NV = ND + 2;
+    double pL[NV], pR[NV], evL, evR;
+    q64::Den rL, rR, kL{}, kR{};
+    prim_core<ND>(e, cL, pL, rL, kL, evL, S, Z);
+    prim_core<ND>(e, cR, pR, rR, kR, evR, S, Z);
+    const double PL = pL[1 + ND], PR = pR[1 + ND];
+    const double aL = q64::root(q64::quo(e.gamma * PL, rL));
+    const double aR = q64::root(q64::quo(e.gamma * PR, rR));
+    const double uL = pL[1 + l];
+    const double uR = pR[1 + l];
+    const double wsL = fmin(uL - aL, uR - aR);
+    const double wsR = fmax(uL + aL, uR + aR);
+    // E and flux of one side's primitives (ek + e, as flux_prim)
+    auto side_flux = [&](const double* p, const q64::Den& k, double* fs) {
+        const double evol = e.kind == EOS_PERFECT_GAS_FAST ? p[1 + ND] * (1.0 / e.gamma_m1) : evol_core(e, p[1 + ND], k);
+        double norm = 0;
+#pragma unroll
+        for (int d = 0; d < ND; ++d) {
+            norm += p[1 + d] * p[1 + d];
+        }
+        const double E = __fma_rn(0.5, p[0] * norm, evol);
+        const double m = p[0] * p[1 + l];
+        fs[0] = m;
+#pragma unroll
+        for (int d = 0; d < ND; ++d) {
+            fs[1 + d] = m * p[1 + d];
+        }
+        fs[1 + l] += p[1 + ND];
+        fs[1 + ND] = p[1 + l] * (E + p[1 + ND]);
+    };
+    zeros = true;
+    if constexpr (RS == RS_HLL) {
+        double fL[NV], fR[NV];
+        side_flux(pL, kL, fL);
+        side_flux(pR, kR, fR);
+        const double nL = fmin(wsL, 0.);
+        const double nR = fmax(wsR, 0.);
+        const q64::Den w = q64::den(nR - nL);
+        S.den(w.b);
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            const double num = (nR * fL[v]) - (nL * fR[v]) + (nL * nR * (cR[v] - cL[v]));
+            f[v] = q64::quo(num, w);
+            Z.add(num);
+            zeros = zeros && q64::within0(num);
+        }
+    } else {
+        const double rcL = pL[0] * (wsL - uL);
+        const double rcR = pR[0] * (wsR - uR);
+        const double un_num = PR - PL + (rcL * uL) - (rcR * uR);
+        // rcL - rcR < 0: quo keeps a zero's sign for positive denominators
+        const q64::Den du = q64::den(-(rcL - rcR));
+        const double ustar = -q64::quo(un_num, du);
+        const double pstar = 1. / 2 * (PL + PR + (rcL * (ustar - uL)) + (rcR * (ustar - uR)));
+        const bool left = ustar > 0;
+        const double Sw = left ? wsL : wsR;
+        double cs[NV], ps[NV], fs[NV];
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            cs[v] = left ? cL[v] : cR[v];
+            ps[v] = left ? pL[v] : pR[v];
+        }
+        side_flux(ps, q64::Den{left ? kL.b : kR.b, left ? kL.y : kR.y}, fs);
+        const double un = ps[1 + l];
+        const q64::Den su = q64::den(Sw - ustar);
+        const double sn = Sw - un;
+        const double un_s = ustar - un;
+        S.den(du.b);
+        S.den(su.b);
+        S.add(sn);
+        Z.add(un_num, un_s);
+        zeros = q64::within0(un_num) && q64::within0(un_s);
+        double rs, Es;
+        if (e.kind == EOS_PERFECT_GAS_FAST) {
+            const double ratio = sn * su.y;
+            rs = cs[0] * ratio;
+            Es = ratio * cs[1 + ND] + un_s * su.y * (ustar * cs[0] * sn + ps[1 + ND]);
+        } else {
+            rs = q64::quo(cs[0] * sn, su);
+            Es = (q64::quo(sn, su) * cs[1 + ND]) + (q64::quo(un_s, su) * ((ustar * cs[0] * sn) + ps[1 + ND]));
+        }
+        const double rsu = rs * ustar;
+        const bool sup = wsL * wsR > 0;
+        f[0] = plain::flux_hllc(fs[0], cs[0], rs, Sw);
+#pragma unroll
+        for (int d = 0; d < ND; ++d) {
+            f[1 + d] = rsu * ps[1 + d];
+        }
+        f[1 + l] = (rsu * ustar) + pstar;
+        f[1 + ND] = plain::flux_hllc(fs[1 + ND], cs[1 + ND], Es, Sw);
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            f[v] = sup ? fs[v] : f[v];
+        }
+    }
+}
+
+template <int ND, int RS>
+__device__ __forceinline__ void riemann_rs(const Eos& e, const double* cL, const double* cR, int l, double* f)
+{
+    q64::Range S(e.consts_ok), Z;
+    bool zeros;
+    riemann_core<ND, RS>(e, cL, cR, l, f, S, Z, zeros);
+    if (!(S.ok() && Z.ok())) {
+        if (!(S.ok() && zeros && prim_zeros<ND>(e, cL) && prim_zeros<ND>(e, cR))) {
+            double lt[ND + 2], rt[ND + 2], ft[ND + 2];
+#pragma unroll
+            for (int v = 0; v < ND + 2; ++v) {
+                lt[v] = cL[v];
+                rt[v] = cR[v];
+            }
+            riemann_slow<ND>(e, RS, lt, rt, l, ft);
+#pragma unroll
+            for (int v = 0; v < ND + 2; ++v) {
+                f[v] = ft[v];
+            }
+        }
+    }
+}
+
+// hydro/riemann_solver.hpp:22-181.  cL/cR: conservative states; l: direction.
+template <int ND>
+__device__ __forceinline__ void riemann(const Eos& e, int solver, const double* cL, const double* cR, int l, double* f)
+{
+    if (e.kind == EOS_RAD_GAS || solver == RS_SPLITTING) {
+        plain::riemann<ND>(e, solver, cL, cR, l, f);
+    } else if (solver == RS_HLL) {
+        riemann_rs<ND, RS_HLL>(e, cL, cR, l, f);
+    } else {
+        riemann_rs<ND, RS_HLLC>(e, cL, cR, l, f);
+    }
 }
 
 // hydro/source_terms.hpp:16-77 (trigonometric factors precomputed on the host

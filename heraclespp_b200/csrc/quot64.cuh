@@ -1,0 +1,141 @@
+// quot64.cuh -- correctly rounded FP64 quotients and square roots without a
+// branch per operation.
+//
+// a / b compiles to a sequence that ends in a branch to a slow path, so two
+// divisions never overlap: each waits out the other's dependency chain, and
+// every quotient of one density repeats the reciprocal.  Here a denominator's
+// reciprocal is formed once (den) and each quotient costs a product and one
+// residual correction (quo), all of it straight-line code that the compiler
+// interleaves freely.  FP64 tile kernels, a branch per division against these:
+// Sod 1024 cells 14.6 -> 7.6 us per step, 2-D KH 2048^2 with a passive scalar
+// 1.51 -> 1.10 ms, 3-D 128^2 x 256 with a passive scalar 5.2 -> 3.2 ms, all
+// with the same bits.
+//
+// Method: Newton's iteration on the hardware's reciprocal approximation, then
+// the residual correction of Markstein (IBM J. Res. Dev. 34, 1990; Cornea,
+// Harrison and Tang, "Scientific Computing on Itanium", 2002, ch. 4): with y
+// the rounded reciprocal of b and q0 = RN(a y), RN(q0 + y RN(a - b q0)) is the
+// rounded quotient.  The square root is the same scheme on the reciprocal
+// square root.  Both need operands far from overflow and underflow: callers
+// gather a group's operands in a Range and fall back to the plain operators
+// for the whole group when one lies outside (numerators may be zero).
+// tests/test_gpu_quot64.py holds the functions built on them to the CPU's
+// operators, bit for bit, over all exponents.
+#pragma once
+
+#include <cstdint>
+
+namespace hcl::q64 {
+
+// Operands of a group must lie within 2^+-300: quotients then stay within
+// 2^+-600 (squares and products of two within 2^+-900) and a residual, 2^-106
+// of its numerator at the least, stays normal.
+constexpr int kExp = 300;
+
+// The high word of a double read as a float orders like the double's
+// magnitude (sign, the upper eight exponent bits, then the rest); infinities
+// and NaNs read as float NaNs.
+__device__ __forceinline__ float hi_float(double a)
+{
+    return __int_as_float(__double2hiint(a));
+}
+__device__ __forceinline__ float lo_bound()
+{
+    return __int_as_float((1023 - kExp) << 20);
+}
+__device__ __forceinline__ float hi_bound()
+{
+    return __int_as_float((1023 + kExp) << 20);
+}
+__device__ __forceinline__ bool within(double a)
+{
+    const float f = fabsf(hi_float(a));
+    return f >= lo_bound() && f <= hi_bound();
+}
+__device__ __forceinline__ bool within0(double a)
+{
+    return within(a) || a == 0.0;
+}
+// The reciprocal iteration stops one unit short where the significand of b is
+// all ones (the theorem's known exception: 1 / (2 - 2^-52) lies next to a
+// midpoint); a low word of ones sends those to the plain operators.
+__device__ __forceinline__ bool den_ok(double b)
+{
+    return within(b) && __double2loint(b) != -1;
+}
+
+// The operands of a group, gathered at half an instruction per bound and
+// operand (three-input minimum and maximum, NaN-propagating).
+struct Range {
+    float mn, mx;
+    unsigned ones; // largest low word of the denominators
+
+    __device__ __forceinline__ explicit Range(bool good = true) : mn(good ? 1.f : 0.f), mx(1.f), ones(0u) {}
+    __device__ __forceinline__ void add(double a)
+    {
+        const float f = fabsf(hi_float(a));
+        asm("min.NaN.f32 %0, %0, %1;" : "+f"(mn) : "f"(f));
+        asm("max.NaN.f32 %0, %0, %1;" : "+f"(mx) : "f"(f));
+    }
+    __device__ __forceinline__ void add(double a, double b)
+    {
+        const float f = fabsf(hi_float(a)), g = fabsf(hi_float(b));
+        asm("min.NaN.f32 %0, %0, %1, %2;" : "+f"(mn) : "f"(f), "f"(g));
+        asm("max.NaN.f32 %0, %0, %1, %2;" : "+f"(mx) : "f"(f), "f"(g));
+    }
+    // low words of denominators added elsewhere
+    __device__ __forceinline__ void low(double b)
+    {
+        ones = max(ones, (unsigned)__double2loint(b));
+    }
+    __device__ __forceinline__ void den(double b)
+    {
+        add(b);
+        low(b);
+    }
+    __device__ __forceinline__ bool ok() const
+    {
+        return mn >= lo_bound() && mx <= hi_bound() && ones != 0xffffffffu;
+    }
+};
+
+struct Den {
+    double b; // the denominator
+    double y; // its rounded reciprocal
+};
+
+__device__ __forceinline__ Den den_from(double b, double y0)
+{
+    return Den{b, __fma_rn(y0, __fma_rn(-b, y0, 1.0), y0)};
+}
+__device__ __forceinline__ Den den(double b)
+{
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    y = __fma_rn(y, __fma_rn(-b, y, 1.0), y);
+    return den_from(b, y);
+}
+// a / d.b; the residual is formed as b q0 - a so that a zero numerator keeps
+// its sign (d.b > 0)
+__device__ __forceinline__ double quo(double a, const Den& d)
+{
+    const double q = __dmul_rn(a, d.y);
+    return __fma_rn(-__fma_rn(d.b, q, -a), d.y, q);
+}
+
+__device__ __forceinline__ double root(double x)
+{
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    double g = __dmul_rn(x, y);
+    double h = __dmul_rn(0.5, y);
+    double r = __fma_rn(-h, g, 0.5);
+    g = __fma_rn(g, r, g);
+    h = __fma_rn(h, r, h);
+    r = __fma_rn(-h, g, 0.5);
+    g = __fma_rn(g, r, g);
+    h = __fma_rn(h, r, h);
+    return __fma_rn(__fma_rn(-g, g, x), h, g);
+}
+
+} // namespace hcl::q64

@@ -19,12 +19,11 @@ std::atomic<int64_t> g_launches{0};
 namespace {
 
 constexpr int kThreads = 256;
-// The two heaviest stage kernels (Hancock predictor, Godunov update: long FP64
-// dependency chains in the reference's order, 130-140 registers unbounded)
-// ask for three CTAs per SM; the extra warps hide the chains' latency (KH
-// 2048^2 FP64 stage-composed step with one passive scalar 3.81 -> 2.61 ms,
-// two CTAs per SM 2.68 ms; the same bits).
-constexpr int kHeavyMinBlocks = 3;
+// The two heaviest stage kernels (Hancock predictor, Godunov update) ask for
+// two CTAs per SM: three steps of 120 x 100 x 70 through the stage entry
+// points take 3.06 ms unbounded, 2.68 ms at two CTAs, 2.64 ms at three, which
+// spill 2.7 KB per thread; with a branch per division (three CTAs) 3.04 ms.
+constexpr int kHeavyMinBlocks = 2;
 
 struct Box {
     int b[3];
@@ -154,9 +153,10 @@ __global__ void k_face_recon(GridDev g, Box bx, const double* __restrict__ var, 
             const double dl_p = (ki * g.dx[0][i + ki]) + (kj * g.dx[1][j + kj]) + (kk * g.dx[2][k + kk]);
             const double vp = var[lidx(g, i + ki, j + kj, k + kk)];
             const double vm = var[lidx(g, i - ki, j - kj, k - kk)];
-            const double slope = exact::slope(g.limiter, (vp - v) / ((dl + dl_p) / 2), (v - vm) / ((dl_m + dl) / 2));
-            rec[c + 2 * g.N * idim] = v - ((dl / 2) * slope);
-            rec[c + g.N + 2 * g.N * idim] = v + ((dl / 2) * slope);
+            double lo, hi;
+            exact::faces<1>(EOS_PERFECT_GAS, g.limiter, false, &vm, &v, &vp, dl_m, dl, dl_p, &lo, &hi);
+            rec[c + 2 * g.N * idim] = lo;
+            rec[c + g.N + 2 * g.N * idim] = hi;
         }
     }
 }
