@@ -737,6 +737,11 @@ int hcl_create(const hcl_config* cfg, hcl_handle** out)
         return bail(fail(HCL_ERR_CUDA, "cudaStreamCreate failed"));
     }
     GridDev& g = h->g;
+    if (cfg->precision == HCL_FP64) {
+        hcl::fused::configure_march_exact(g);
+    } else if (cfg->precision == HCL_FP64_FAST) {
+        hcl::fused::configure_march_fast(g);
+    }
     for (int d = 0; d < 3; ++d) {
         if ((rc = upload(&h->dx_nodes[d], h->hx[d])) || (rc = upload(&h->ddx[d], h->hdx[d])) ||
             (rc = upload(&h->dxc[d], h->hxc[d]))) {

@@ -28,7 +28,11 @@ void step_exact(const GridDev& g, const StateDev& in, const StateDev& out, StepC
         FusedLauncher<1, true, 128, 1, 1>::launch(g, in, out, ctl, rp, slot, out_buf, s);
         break;
     case 2:
-        FusedLauncher<2, true, 16, 16, 1>::launch(g, in, out, ctl, rp, slot, out_buf, s);
+        if (march2d64_valid(g)) {
+            march2d_exact(g, in, out, ctl, rp, slot, out_buf, s);
+        } else {
+            FusedLauncher<2, true, 16, 16, 1>::launch(g, in, out, ctl, rp, slot, out_buf, s);
+        }
         break;
     default:
         // 8x8x4 tiles (less halo than 8x4x4: RT 256^2 x 512 39.9 -> 33.9 ms per

@@ -28,7 +28,11 @@ void step_fast64(const GridDev& g, const StateDev& in, const StateDev& out, Step
         FusedLauncher<1, true, 128, 1, 1>::launch_kind<EOS_PERFECT_GAS_FAST>(g, in, out, ctl, rp, slot, out_buf, s);
         break;
     case 2:
-        FusedLauncher<2, true, 16, 16, 1>::launch_kind<EOS_PERFECT_GAS_FAST>(g, in, out, ctl, rp, slot, out_buf, s);
+        if (march2d64_valid(g)) {
+            march2d_fast(g, in, out, ctl, rp, slot, out_buf, s);
+        } else {
+            FusedLauncher<2, true, 16, 16, 1>::launch_kind<EOS_PERFECT_GAS_FAST>(g, in, out, ctl, rp, slot, out_buf, s);
+        }
         break;
     default:
         if (big_tile_3d_fits_fast(g)) {

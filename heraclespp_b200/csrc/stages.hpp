@@ -115,6 +115,15 @@ bool strip2d_tma_eligible(const GridDev& g);
 // stride is not a multiple of 16 bytes.
 bool encode_tile_map(const GridDev& g, const StateDev& st, int nv, const int box[3], CUtensorMap* map);
 void configure_exact();
+// FP64 march kernels (march64_exact.cu, march64_fast.cu): the step of the
+// grids march2d64_valid() accepts, and their once-per-device set-up
+bool march2d64_valid(const GridDev& g);
+void configure_march_exact(const GridDev& g);
+void configure_march_fast(const GridDev& g);
+void march2d_exact(const GridDev& g, const StateDev& in, const StateDev& out, StepCtl* ctl, const RunParamsDev& rp,
+                   int slot, int out_buf, cudaStream_t s);
+void march2d_fast(const GridDev& g, const StateDev& in, const StateDev& out, StepCtl* ctl, const RunParamsDev& rp,
+                  int slot, int out_buf, cudaStream_t s);
 void configure_mixed();
 int conservation_partials_doubles(int ndim);
 
