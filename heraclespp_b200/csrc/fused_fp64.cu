@@ -37,7 +37,9 @@ void step_exact(const GridDev& g, const StateDev& in, const StateDev& out, StepC
     default:
         // 8x8x4 tiles (less halo than 8x4x4: RT 256^2 x 512 39.9 -> 33.9 ms per
         // step) unless the passive scalars need the smaller tile's shared memory
-        if (big_tile_3d_fits(g)) {
+        if (march3d64_valid(g)) {
+            march3d_exact(g, in, out, ctl, rp, slot, out_buf, s);
+        } else if (big_tile_3d_fits(g)) {
             FusedLauncher<3, true, 8, 8, 4>::launch(g, in, out, ctl, rp, slot, out_buf, s);
         } else {
             FusedLauncher<3, true, 8, 4, 4>::launch(g, in, out, ctl, rp, slot, out_buf, s);

@@ -35,7 +35,9 @@ void step_fast64(const GridDev& g, const StateDev& in, const StateDev& out, Step
         }
         break;
     default:
-        if (big_tile_3d_fits_fast(g)) {
+        if (march3d64_valid(g)) {
+            march3d_fast(g, in, out, ctl, rp, slot, out_buf, s);
+        } else if (big_tile_3d_fits_fast(g)) {
             FusedLauncher<3, true, 8, 8, 4>::launch_kind<EOS_PERFECT_GAS_FAST>(g, in, out, ctl, rp, slot, out_buf, s);
         } else {
             FusedLauncher<3, true, 8, 4, 4>::launch_kind<EOS_PERFECT_GAS_FAST>(g, in, out, ctl, rp, slot, out_buf, s);

@@ -1,6 +1,7 @@
 // march64_fast.cu -- the FP64 march kernels in the fast FP64 forms (compiled
-// with FMA contraction; see march2d64.cuh).
+// with FMA contraction; see march2d64.cuh and march3d64.cuh).
 #include "march2d64.cuh"
+#include "march3d64.cuh"
 #include "stages.hpp"
 
 namespace hcl::fused {
@@ -9,6 +10,10 @@ void configure_march_fast(const GridDev& g)
 {
     if (march2d64_valid(g)) {
         march64_pick(g, [](auto lim, auto rs) { march2d64_configure_t<decltype(lim)::value, decltype(rs)::value, EOS_PERFECT_GAS_FAST>(); });
+    } else if (march3d64_valid(g)) {
+        march64_pick(g, [](auto lim, auto rs) {
+            march3d64_configure_t<decltype(lim)::value, decltype(rs)::value, EOS_PERFECT_GAS_FAST>();
+        });
     }
 }
 
@@ -17,6 +22,14 @@ void march2d_fast(const GridDev& g, const StateDev& in, const StateDev& out, Ste
 {
     march64_pick(g, [&](auto lim, auto rs) {
         march2d64_launch_t<decltype(lim)::value, decltype(rs)::value, EOS_PERFECT_GAS_FAST>(g, in, out, ctl, rp, slot, out_buf, s);
+    });
+}
+
+void march3d_fast(const GridDev& g, const StateDev& in, const StateDev& out, StepCtl* ctl, const RunParamsDev& rp,
+                 int slot, int out_buf, cudaStream_t s)
+{
+    march64_pick(g, [&](auto lim, auto rs) {
+        march3d64_launch_t<decltype(lim)::value, decltype(rs)::value, EOS_PERFECT_GAS_FAST>(g, in, out, ctl, rp, slot, out_buf, s);
     });
 }
 

@@ -118,10 +118,15 @@ void configure_exact();
 // FP64 march kernels (march64_exact.cu, march64_fast.cu): the step of the
 // grids march2d64_valid() accepts, and their once-per-device set-up
 bool march2d64_valid(const GridDev& g);
+bool march3d64_valid(const GridDev& g);
 void configure_march_exact(const GridDev& g);
 void configure_march_fast(const GridDev& g);
 void march2d_exact(const GridDev& g, const StateDev& in, const StateDev& out, StepCtl* ctl, const RunParamsDev& rp,
                    int slot, int out_buf, cudaStream_t s);
+void march3d_exact(const GridDev& g, const StateDev& in, const StateDev& out, StepCtl* ctl, const RunParamsDev& rp,
+                   int slot, int out_buf, cudaStream_t s);
+void march3d_fast(const GridDev& g, const StateDev& in, const StateDev& out, StepCtl* ctl, const RunParamsDev& rp,
+                  int slot, int out_buf, cudaStream_t s);
 void march2d_fast(const GridDev& g, const StateDev& in, const StateDev& out, StepCtl* ctl, const RunParamsDev& rp,
                   int slot, int out_buf, cudaStream_t s);
 void configure_mixed();

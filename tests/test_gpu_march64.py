@@ -1,5 +1,6 @@
-"""The FP64 march kernels (Cartesian 2-D) against the oracle: sizes at
-the edges of their tiles (28-column warps), one cell less and more, and the smallest grids (two cells)."""
+"""The FP64 march kernels (Cartesian 2-D and 3-D) against the oracle: sizes at
+the edges of their tiles (28-column warps in 2-D, 30 x 10 column blocks in
+3-D), one cell less and more, and the smallest grids (two cells)."""
 import numpy as np
 import pytest
 
@@ -10,7 +11,9 @@ from oracle import Oracle
 pytestmark = pytest.mark.gpu
 
 BC2 = [["Periodic"] * 4, ["NullGradient", "Reflexive", "Reflexive", "NullGradient"]]
+BC3 = [["Periodic"] * 6, ["NullGradient", "Reflexive", "Reflexive", "NullGradient", "Reflexive", "NullGradient"]]
 G2D = [([2, 2], 0), ([27, 5], 1), ([28, 3], 0), ([29, 34], 1), ([57, 41], 1)]
+G3D = [([2, 2, 2], 0), ([29, 9, 3], 1), ([30, 10, 7], 0), ([31, 11, 12], 1), ([33, 21, 5], 1)]
 PHYS = [("VanLeer", "HLLC"), ("Minmod", "HLL"), ("VanAlbada", "Low Mach"), ("Constant", "HLLC")]
 
 
@@ -31,10 +34,10 @@ def flow(o, seed):
 
 
 @pytest.mark.parametrize("lim,rs", PHYS)
-@pytest.mark.parametrize("nx,b", G2D)
+@pytest.mark.parametrize("nx,b", G2D + G3D)
 def test_march_matches_oracle(nx, b, lim, rs):
     nd = len(nx)
-    kw = dict(gamma=1.4, limiter=lim, riemann=rs, bc=BC2[b], xmax=(1.0, 0.7, 1.3),
+    kw = dict(gamma=1.4, limiter=lim, riemann=rs, bc=(BC2 if nd == 2 else BC3)[b], xmax=(1.0, 0.7, 1.3),
               g=(0.03, -0.05, 0.02) if b else (0.0, 0.0, 0.0))
     o = Oracle(nd, nx, **kw)
     prim = flow(o, 5 + nx[0])
