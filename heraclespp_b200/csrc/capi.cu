@@ -99,10 +99,11 @@ struct hcl_handle {
     hcl_config cfg{};
     GridDev g{};
     // host grid arrays
-    std::vector<double> hx[3], hdx[3], hxc[3], hds, hdv, hgr, hcot, hsin1, hsinxc1;
+    std::vector<double> hx[3], hdx[3], hxc[3], hds, hdv, hgr, hcot, hsin1, hsinxc1, hshell_dv;
     // device grid arrays
     double *dx_nodes[3] = {}, *ddx[3] = {}, *dxc[3] = {}, *dds = nullptr, *ddv = nullptr, *dgr = nullptr;
     double *dcot = nullptr, *dsin1 = nullptr, *dsinxc1 = nullptr;
+    double* dshell_dv = nullptr;  // InternalMassGravity: the shells' volumes
     double* grav_shell = nullptr; // InternalMassGravity: shell means of rho (nx0 + ng)
     // stage-path scratch (MUSCLHancockHydroReconstruction's P_rec/u_rec, fx_rec_old)
     double *u_rec = nullptr, *P_rec = nullptr, *fx_rec_old = nullptr;
@@ -191,6 +192,7 @@ void free_handle(hcl_handle* h)
     cudaFree(h->ddv);
     cudaFree(h->dgr);
     cudaFree(h->grav_shell);
+    cudaFree(h->dshell_dv);
     cudaFree(h->dcot);
     cudaFree(h->dsin1);
     cudaFree(h->dsinxc1);
@@ -301,6 +303,18 @@ void build_grid_host(hcl_handle* h)
         }
     } else if (c.gravity == HCL_GRAVITY_INTERNAL_MASS) {
         h->hgr.assign(n[0], 0.0); // filled from the density (refresh_gravity)
+        // the shells' volumes (gravity.cpp:59-128), j outer, k inner
+        const int g1 = nd >= 2 ? c.nghost : 0, g2 = nd >= 3 ? c.nghost : 0;
+        h->hshell_dv.assign((size_t)nx[0] + c.nghost, 0.0);
+        for (int i = 0; i < nx[0] + c.nghost; ++i) {
+            double sd = 0;
+            for (int j = 0; j < nx[1]; ++j) {
+                for (int k = 0; k < nx[2]; ++k) {
+                    sd += h->hdv[(size_t)(i + c.nghost + (int64_t)n[0] * (j + g1 + (int64_t)n[1] * (k + g2)))];
+                }
+            }
+            h->hshell_dv[i] = sd;
+        }
     }
     // spherical trig factors per index (source_terms.hpp:38, :58-59, time_step.hpp:67)
     h->hcot.assign(n[1], 0.0);
@@ -757,9 +771,10 @@ int hcl_create(const hcl_config* cfg, hcl_handle** out)
         return bail(rc);
     }
     if (h->cfg.gravity == HCL_GRAVITY_INTERNAL_MASS &&
-        (rc = dalloc(&h->grav_shell, (size_t)(g.nx[0] + g.ng)))) {
+        ((rc = dalloc(&h->grav_shell, (size_t)(g.nx[0] + g.ng))) || (rc = upload(&h->dshell_dv, h->hshell_dv)))) {
         return bail(rc);
     }
+    g.shell_dv = h->dshell_dv;
     g.ds = h->dds;
     g.dv = h->ddv;
     g.g_r = h->dgr;

@@ -55,6 +55,7 @@ struct GridDev {
     const double* ds;     // N*3
     const double* dv;     // N
     const double* g_r;    // point-mass / internal-mass g(i), n[0]
+    const double* shell_dv; // internal-mass gravity: sum of dv over each shell's interior (j, k)
     // geometry helpers precomputed on the host for spherical runs (per index):
     const double* cot_mid1;   // cos((x1_j+x1_{j+1})/2)/sin(...) per j, source_terms.hpp:38
     const double* sin1;       // sin(x1_j) per node j, source_terms.hpp:58-59

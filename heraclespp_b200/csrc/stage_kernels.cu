@@ -805,56 +805,103 @@ void dispatch_nd(int nd, F&& f)
     }
 }
 
-// InternalMassGravity (gravity.cpp:59-128), one CTA: each thread sums the
-// density of one radial shell over the interior (j, k) (j outer, k inner),
-// thread 0 runs the enclosed-mass sum outwards from the central mass, then
-// every thread turns its cells' enclosed mass into g = -G M / xc^2.  rho has
-// rows of `pitch` doubles (n0 for the reference layout); shell: nx0 + ng
-// doubles of scratch; g_r: n0 doubles (the handle's radial table).
-__global__ void k_internal_mass_gravity(GridDev g, const double* __restrict__ rho, int pitch, double central_mass,
-                                        double* __restrict__ shell, double* __restrict__ g_r)
+// InternalMassGravity (gravity.cpp:59-128): the shell means of rho, then the
+// enclosed mass and the radial table g = -G M / xc^2.  rho has rows of `pitch`
+// doubles (n0 for the reference layout); shell: nx0 + ng doubles of scratch;
+// g_r: n0 doubles (the handle's radial table).
+//
+// A shell's mean is a sum over (j, k) in a fixed order (j outer, k inner), one
+// dependent addition per cell, so its floor is the addition's latency: 3200
+// cells of a 96 x 64 x 50 grid, ~15 us.  A CTA sums 32 shells with one warp
+// while its other warps bring in the next chunk's products rho dv through
+// shared memory; with one thread per shell loading for itself each addition
+// waited out its own loads (954 us).  The shells' volumes do not change and
+// come from the host (g.shell_dv).
+constexpr int kShellWarps = 16;
+constexpr int kShellChunk = 96; // 2 buffers x 96 x 32 doubles = 48 KB
+__global__ void __launch_bounds__(32 * kShellWarps) k_shell_means(GridDev g, const double* __restrict__ rho, int pitch,
+                                                                  double* __restrict__ shell)
 {
-    const int ng = g.ng;
-    const int nsh = g.nx[0] + ng;
-    const int g1 = g.ndim >= 2 ? ng : 0;
-    const int g2 = g.ndim >= 3 ? ng : 0;
-    for (int i = threadIdx.x; i < nsh; i += blockDim.x) {
-        double sm = 0;
-        double sd = 0;
-        for (int j = 0; j < g.nx[1]; ++j) {
-            for (int k = 0; k < g.nx[2]; ++k) {
-                const int64_t id = lidx(g, i + ng, j + g1, k + g2);
-                const int64_t ir = ((int64_t)(k + g2) * g.n[1] + (j + g1)) * pitch + (i + ng);
-                sm += rho[ir] * g.dv[id];
-                sd += g.dv[id];
+    __shared__ double buf[2][kShellChunk][32];
+    const int lane = threadIdx.x & 31;
+    const int w = threadIdx.x >> 5;
+    const int nsh = g.nx[0] + g.ng;
+    const int sh = blockIdx.x * 32 + lane;
+    const int i = min(sh, nsh - 1) + g.ng;
+    const int g1 = g.ndim >= 2 ? g.ng : 0;
+    const int g2 = g.ndim >= 3 ? g.ng : 0;
+    const int nk = g.nx[2];
+    const int64_t count = (int64_t)g.nx[1] * nk;
+    auto load = [&](int64_t c0, int b, int first, int nw) {
+        for (int r = first; r < kShellChunk && c0 + r < count; r += nw) {
+            const int64_t c = c0 + r;
+            const int j = (int)(c / nk) + g1;
+            const int k = (int)(c % nk) + g2;
+            buf[b][r][lane] = rho[((int64_t)k * g.n[1] + j) * pitch + i] * g.dv[lidx(g, i, j, k)];
+        }
+    };
+    load(0, 0, w, kShellWarps);
+    __syncthreads();
+    double sm = 0;
+    int b = 0;
+    for (int64_t c0 = 0; c0 < count; c0 += kShellChunk, b ^= 1) {
+        if (w > 0) {
+            load(c0 + kShellChunk, b ^ 1, w - 1, kShellWarps - 1);
+        } else if (count - c0 >= kShellChunk) {
+#pragma unroll 16
+            for (int r = 0; r < kShellChunk; ++r) {
+                sm += buf[b][r][lane];
+            }
+        } else {
+            for (int r = 0; r < (int)(count - c0); ++r) {
+                sm += buf[b][r][lane];
             }
         }
-        shell[i] = sm / sd;
+        __syncthreads();
     }
-    __syncthreads();
+    if (w == 0 && sh < nsh) {
+        shell[sh] = sm / g.shell_dv[sh];
+    }
+}
+
+// The enclosed mass runs outwards from the central mass in order; its terms
+// are formed in parallel, a chunk of radii at a time.
+constexpr int kMassThreads = 256;
+__global__ void __launch_bounds__(kMassThreads) k_internal_mass_gravity(GridDev g, double central_mass,
+                                                                        const double* __restrict__ shell,
+                                                                        double* __restrict__ g_r)
+{
+    __shared__ double term[kMassThreads];
+    const int ng = g.ng;
     const double* x0 = g.x[0];
     const double* xc = g.xc[0];
-    if (threadIdx.x == 0) {
-        const double vol_s3 = 4 * kPi / 3;
-        for (int i = 0; i < ng; ++i) {
-            g_r[i] = central_mass;
-        }
-        double partial = 0;
-        for (int i = ng; i < g.nx[0] + 2 * ng; ++i) {
+    const double vol_s3 = 4 * kPi / 3;
+    double partial = 0;
+    for (int c0 = 0; c0 < g.n[0]; c0 += kMassThreads) {
+        const int i = c0 + threadIdx.x;
+        if (i < ng) {
+            term[threadIdx.x] = central_mass;
+        } else if (i < g.n[0]) {
             const int off = i - ng;
             const double x3 = x0[i] * x0[i] * x0[i];
-            if (i == ng) {
-                partial += central_mass + (vol_s3 * ((xc[i] * xc[i] * xc[i]) - x3) * shell[off]);
-            } else {
-                partial += (vol_s3 * (x3 - (xc[i - 1] * xc[i - 1] * xc[i - 1])) * shell[off - 1]) +
-                           (vol_s3 * ((xc[i] * xc[i] * xc[i]) - x3) * shell[off]);
-            }
-            g_r[i] = partial;
+            const double up = vol_s3 * ((xc[i] * xc[i] * xc[i]) - x3) * shell[off];
+            term[threadIdx.x] =
+                i == ng ? central_mass + up
+                        : (vol_s3 * (x3 - (xc[i - 1] * xc[i - 1] * xc[i - 1])) * shell[off - 1]) + up;
         }
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < g.n[0]; i += blockDim.x) {
-        g_r[i] = -kG * g_r[i] / (xc[i] * xc[i]);
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            const int m = min(kMassThreads, g.n[0] - c0);
+            for (int r = c0 < ng ? ng - c0 : 0; r < m; ++r) {
+                partial += term[r];
+                term[r] = partial;
+            }
+        }
+        __syncthreads();
+        if (i < g.n[0]) {
+            g_r[i] = -kG * term[threadIdx.x] / (xc[i] * xc[i]);
+        }
+        __syncthreads();
     }
 }
 
@@ -968,8 +1015,9 @@ void pressure_fix(const GridDev& g, double dt, double eps, const double* rho, co
 void internal_mass_gravity(const GridDev& g, const double* rho, int pitch, double central_mass, double* shell,
                            double* g_r, cudaStream_t s)
 {
-    k_internal_mass_gravity<<<1, 256, 0, s>>>(g, rho, pitch, central_mass, shell, g_r);
-    ++g_launches;
+    k_shell_means<<<(g.nx[0] + g.ng + 31) / 32, 32 * kShellWarps, 0, s>>>(g, rho, pitch, shell);
+    k_internal_mass_gravity<<<1, kMassThreads, 0, s>>>(g, central_mass, shell, g_r);
+    g_launches += 2;
 }
 
 void boundaries(const GridDev& g, double* rho, double* rhou, double* E, double* fx, cudaStream_t s)
