@@ -1528,6 +1528,42 @@ static int run_stage_loop(hcl_handle* h, const hcl_run_params* p, hcl_run_result
     return HCL_OK;
 }
 
+// The state and the result of a run whose steps are all launched.
+static int finish_run(hcl_handle* h, hcl_run_result* r)
+{
+    StepCtl ctl;
+    int rc;
+    if ((rc = read_ctl(h, &ctl))) {
+        return rc;
+    }
+    const int q = (int)(h->counter & 1);
+    const bool stop = ctl.stop[q] || ctl.err;
+    h->cur = stop ? ctl.final_buf : q;
+    h->stopped = stop ? 1 : 0;
+    if ((rc = refresh_gravity(h))) {
+        return rc;
+    }
+    if (r) {
+        r->t = ctl.t[q];
+        r->iter = ctl.iter[q];
+        r->status = ctl.err;
+        r->bad_cell = ctl.bad_cell == ~0ull ? -1 : (int64_t)ctl.bad_cell;
+        r->finished = ctl.stop[q] ? 1 : 0;
+        r->last_dt = ctl.last_dt;
+    }
+    if (ctl.err == HCL_ERR_INVALID_STATE) {
+        return fail(HCL_ERR_INVALID_STATE, "detected invalid volumic internal energy at cell %lld",
+                    (long long)(ctl.bad_cell == ~0ull ? -1 : (long long)ctl.bad_cell));
+    }
+    if (ctl.err == HCL_ERR_NEGATIVE_DT) {
+        return fail(HCL_ERR_NEGATIVE_DT, "Error: the time step is negative");
+    }
+    if (ctl.err == HCL_ERR_TIMEOUT) {
+        return fail(HCL_ERR_TIMEOUT, "a bounded device-side wait for a staged state row gave up");
+    }
+    return HCL_OK;
+}
+
 int hcl_run(hcl_handle* h, const hcl_run_params* p, hcl_run_result* r)
 {
     HCL_CHECK_HANDLE(h);
@@ -1597,6 +1633,35 @@ int hcl_run(hcl_handle* h, const hcl_run_params* p, hcl_run_result* r)
                                  h->stream));
         rp.dts = h->d_dts;
     }
+    if (h->cfg.precision != HCL_FP32_MIXED && hcl::fused::march1d64_valid(h->g)) {
+        // one launch carries many steps and ends early when the run stops
+        constexpr int kMaxSteps = 4096;
+        for (int done = 0;;) {
+            const int m = nsteps > 0 ? std::min(nsteps - done, kMaxSteps) : kMaxSteps;
+            const int slot = (int)(h->counter % 6);
+            if (h->cfg.precision == HCL_FP64) {
+                hcl::fused::march1d_exact(h->g, h->st[0], h->st[1], h->ctl, rp, slot, m, h->stream);
+            } else {
+                hcl::fused::march1d_fast(h->g, h->st[0], h->st[1], h->ctl, rp, slot, m, h->stream);
+            }
+            HCL_LAUNCH_CHECK();
+            h->counter += m;
+            done += m;
+            if (nsteps > 0) {
+                if (done >= nsteps) {
+                    break;
+                }
+                continue;
+            }
+            if ((rc = read_ctl(h, &ctl))) {
+                return rc;
+            }
+            if (ctl.stop[h->counter & 1] || ctl.errflag[h->counter & 1] || ctl.err) {
+                break;
+            }
+        }
+        return finish_run(h, r);
+    }
     const int K = p->graph_chunk > 0 ? (p->graph_chunk + 5) / 6 * 6 : 60;
     const int shape = h->mixed_shape < 0 ? 0 : h->mixed_shape;
     // A run of a fixed step count replays the largest of these graphs that
@@ -1663,35 +1728,7 @@ int hcl_run(hcl_handle* h, const hcl_run_params* p, hcl_run_result* r)
             finished = ctl.stop[h->counter & 1] || ctl.errflag[h->counter & 1] || ctl.err;
         }
     }
-    if ((rc = read_ctl(h, &ctl))) {
-        return rc;
-    }
-    const int q = (int)(h->counter & 1);
-    const bool stop = ctl.stop[q] || ctl.err;
-    h->cur = stop ? ctl.final_buf : q;
-    h->stopped = stop ? 1 : 0;
-    if ((rc = refresh_gravity(h))) {
-        return rc;
-    }
-    if (r) {
-        r->t = ctl.t[q];
-        r->iter = ctl.iter[q];
-        r->status = ctl.err;
-        r->bad_cell = ctl.bad_cell == ~0ull ? -1 : (int64_t)ctl.bad_cell;
-        r->finished = ctl.stop[q] ? 1 : 0;
-        r->last_dt = ctl.last_dt;
-    }
-    if (ctl.err == HCL_ERR_INVALID_STATE) {
-        return fail(HCL_ERR_INVALID_STATE, "detected invalid volumic internal energy at cell %lld",
-                    (long long)(ctl.bad_cell == ~0ull ? -1 : (long long)ctl.bad_cell));
-    }
-    if (ctl.err == HCL_ERR_NEGATIVE_DT) {
-        return fail(HCL_ERR_NEGATIVE_DT, "Error: the time step is negative");
-    }
-    if (ctl.err == HCL_ERR_TIMEOUT) {
-        return fail(HCL_ERR_TIMEOUT, "a bounded device-side wait for a staged state row gave up");
-    }
-    return HCL_OK;
+    return finish_run(h, r);
 }
 
 int hcl_step_fixed_dt(hcl_handle* h, double dt, void* stream)

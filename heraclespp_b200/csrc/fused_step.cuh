@@ -100,28 +100,25 @@ struct Decision {
     int ioid_next;
 };
 
-__device__ __forceinline__ Decision decide(const StepCtl* ctl, int slot, const RunParamsDev& rp)
+// The step after (t, iter) with the output counters toid, ioid, 1/dt = inv_bits.
+__device__ __forceinline__ Decision decide_values(double t, int iter, int toid, int ioid, unsigned long long inv_bits,
+                                                  const RunParamsDev& rp)
 {
     Decision d;
-    const int p = slot & 1;
-    d.t = ctl->t[p];
-    d.iter = ctl->iter[p];
-    d.noop = ctl->stop[p] || ctl->errflag[p];
+    d.t = t;
+    d.iter = iter;
+    d.noop = 0;
     d.stop = 0;
     d.neg_dt = 0;
-    d.toid_next = ctl->time_output_id[p];
-    d.ioid_next = ctl->iter_output_id[p];
-    d.dt = 0;
-    if (d.noop) {
-        return d;
-    }
+    d.toid_next = toid;
+    d.ioid_next = ioid;
     double dt;
     if (rp.fixed_dt == 1) {
         dt = rp.dts[d.iter];
     } else if (rp.fixed_dt == 2) {
         dt = rp.dt_value;
     } else {
-        const double inv = __longlong_as_double((long long)ctl->inv_dt_bits[slot % 3]);
+        const double inv = __longlong_as_double((long long)inv_bits);
         dt = rp.cfl * (1 / inv); // main.cpp:355, time_step.hpp:82
     }
     if (rp.iter_frequency > 0) { // main.cpp:358-364
@@ -149,6 +146,16 @@ __device__ __forceinline__ Decision decide(const StepCtl* ctl, int slot, const R
     }
     d.dt = dt;
     return d;
+}
+
+__device__ __forceinline__ Decision decide(const StepCtl* ctl, int slot, const RunParamsDev& rp)
+{
+    const int p = slot & 1;
+    if (ctl->stop[p] || ctl->errflag[p]) {
+        return Decision{0.0, ctl->t[p], ctl->iter[p], 1, 0, 0, ctl->time_output_id[p], ctl->iter_output_id[p]};
+    }
+    return decide_values(ctl->t[p], ctl->iter[p], ctl->time_output_id[p], ctl->iter_output_id[p],
+                         ctl->inv_dt_bits[slot % 3], rp);
 }
 
 __device__ __forceinline__ int64_t sidx(const StateDev& st, int n1, int i, int j, int k)
@@ -580,26 +587,26 @@ __device__ __forceinline__ void fused_step_body(const GridDev& g, const StateDev
                     vp[v] = sp[v * S::NP + lc + lstride[idim]];
                 }
                 exact::faces<NV>(EOSK, g.limiter, g.uniform_cart, vm, vc, vp, dl_m, dl, dl_p, fp[0][idim], fp[1][idim]);
-                continue;
-            }
+            } else {
 #pragma unroll
-            for (int v = 0; v < NV; ++v) {
-                const R vc = sp[v * S::NP + lc];
-                const R vp = sp[v * S::NP + lc + lstride[idim]];
-                const R vm = sp[v * S::NP + lc - lstride[idim]];
-                if (g.uniform_cart) {
-                    // dl/2 * limiter(dR/dl, dL/dl) = limiter(dR, dL)/2 (every limiter
-                    // is positively homogeneous of degree 1)
-                    const float s = 0.5f * fast::limited(g.limiter, vp - vc, vc - vm);
-                    fp[0][idim][v] = vc - s;
-                    fp[1][idim][v] = vc + s;
-                } else {
-                    const float fdl = (float)dl;
-                    const float hR = 2.f * fast::rcp(fdl + (float)dl_p);
-                    const float hL = 2.f * fast::rcp((float)dl_m + fdl);
-                    const float s = 0.5f * fdl * fast::limited(g.limiter, (vp - vc) * hR, (vc - vm) * hL);
-                    fp[0][idim][v] = vc - s;
-                    fp[1][idim][v] = vc + s;
+                for (int v = 0; v < NV; ++v) {
+                    const R vc = sp[v * S::NP + lc];
+                    const R vp = sp[v * S::NP + lc + lstride[idim]];
+                    const R vm = sp[v * S::NP + lc - lstride[idim]];
+                    if (g.uniform_cart) {
+                        // dl/2 * limiter(dR/dl, dL/dl) = limiter(dR, dL)/2 (every limiter
+                        // is positively homogeneous of degree 1)
+                        const float s = 0.5f * fast::limited(g.limiter, vp - vc, vc - vm);
+                        fp[0][idim][v] = vc - s;
+                        fp[1][idim][v] = vc + s;
+                    } else {
+                        const float fdl = (float)dl;
+                        const float hR = 2.f * fast::rcp(fdl + (float)dl_p);
+                        const float hL = 2.f * fast::rcp((float)dl_m + fdl);
+                        const float s = 0.5f * fdl * fast::limited(g.limiter, (vp - vc) * hR, (vc - vm) * hL);
+                        fp[0][idim][v] = vc - s;
+                        fp[1][idim][v] = vc + s;
+                    }
                 }
             }
         }
@@ -1187,7 +1194,12 @@ __device__ __forceinline__ void fused_step_body(const GridDev& g, const StateDev
         // health check (main.cpp:397-425) and CFL of the new state (time_step.hpp:55-77)
         double evol, inv_rho_u[ND], sound;
         if constexpr (EXACT) {
-            exact::state_speeds<ND>(eeos, qn, evol, sound, inv_rho_u);
+            double pr[NV];
+            exact::state_prims<ND>(eeos, qn, evol, sound, pr);
+#pragma unroll
+            for (int d = 0; d < ND; ++d) {
+                inv_rho_u[d] = fabs(pr[1 + d]);
+            }
         } else {
             double r = (double)__frcp_rn((float)qn[0]);
             r = r * (2.0 - qn[0] * r);

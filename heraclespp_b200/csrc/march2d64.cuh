@@ -329,8 +329,9 @@ __device__ __forceinline__ void march2d_strip(const GridDev& g, const double* __
                 qn[3] += dt * gvy * ring[r & 7][2][lane];
             }
             if (out_lane) {
-                double evol, snd, au[2];
-                exact::state_speeds<2>(e, qn, evol, snd, au);
+                double evol, snd, pn[4];
+                exact::state_prims<2>(e, qn, evol, snd, pn);
+                const double au[2] = {fabs(pn[1]), fabs(pn[2])};
                 if (!(evol >= 0.0) && bad_cell < 0) {
                     bad_cell = lidx(g, col, r, 0);
                 }

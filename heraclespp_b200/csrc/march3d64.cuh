@@ -308,8 +308,9 @@ k_march3d64(GridDev g, StateDev in, StateDev out, StepCtl* ctl, RunParamsDev rp,
                         qn[3] += dt * gv[2] * in.q[o];
                         qn[4] += dt * gv[2] * in.q[o + 3 * in.plane];
                     }
-                    double evol, snd, au[3];
-                    exact::state_speeds<3>(e, qn, evol, snd, au);
+                    double evol, snd, pn[5];
+                    exact::state_prims<3>(e, qn, evol, snd, pn);
+                    const double au[3] = {fabs(pn[1]), fabs(pn[2]), fabs(pn[3])};
                     if (!(evol >= 0.0) && bad_cell < 0) {
                         bad_cell = lidx(g, col, row, r);
                     }

@@ -1,15 +1,39 @@
 // march64_exact.cu -- the FP64 march kernels in the reference's arithmetic
-// (compiled with --fmad=false; see march2d64.cuh and march3d64.cuh).
+// (compiled with --fmad=false; see march1d64.cuh, march2d64.cuh and
+// march3d64.cuh).
+#include "march1d64.cuh"
 #include "march2d64.cuh"
 #include "march3d64.cuh"
 #include "stages.hpp"
 
 namespace hcl::fused {
 
-// Cartesian 2-D grids of the perfect gas without scalars or pressure fix
+// Perfect-gas 1-D domains without scalars or pressure fix, with a gravity
+// table that does not change from step to step, up to 16 CTAs' cells
+bool march1d64_valid(const GridDev& g)
+{
+    return g.ndim == 1 && g.eos == EOS_PERFECT_GAS && g.nfx == 0 && !g.pressure_fix &&
+           g.gravity != GRAV_INTERNAL_MASS && g.nx[0] <= kM1MaxCtas * kM1MaxChunk &&
+           march1d64_configure_t<EOS_PERFECT_GAS>();
+}
+
+// Cartesian 2-D grids of the perfect gas without scalars or pressure fix, from
+// more 16 x 16 tiles than one wave of the tile kernel holds (two per SM): a
+// strip is at least four row iterations deep, a single tile is quicker (us per
+// step, tile and march: 256^2 18.3 and 23.5, 400 x 300 32.4 and 29.3, 512^2
+// 59.7 and 45.6)
 bool march2d64_valid(const GridDev& g)
 {
-    return g.ndim == 2 && g.geom == GEOM_CARTESIAN && g.eos == EOS_PERFECT_GAS && g.nfx == 0 && !g.pressure_fix;
+    static PerDevice cache;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const int sms = cache.get(dev, [dev] {
+        int v = 0;
+        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+        return v;
+    });
+    return g.ndim == 2 && g.geom == GEOM_CARTESIAN && g.eos == EOS_PERFECT_GAS && g.nfx == 0 && !g.pressure_fix &&
+           (int64_t)((g.nx[0] + 15) / 16) * ((g.nx[1] + 15) / 16) > 2 * sms;
 }
 
 // Cartesian 3-D grids, the same
@@ -20,13 +44,21 @@ bool march3d64_valid(const GridDev& g)
 
 void configure_march_exact(const GridDev& g)
 {
-    if (march2d64_valid(g)) {
+    if (g.ndim == 1) {
+        march1d64_configure_t<EOS_PERFECT_GAS>();
+    } else if (march2d64_valid(g)) {
         march64_pick(g, [](auto lim, auto rs) { march2d64_configure_t<decltype(lim)::value, decltype(rs)::value, EOS_PERFECT_GAS>(); });
     } else if (march3d64_valid(g)) {
         march64_pick(g, [](auto lim, auto rs) {
             march3d64_configure_t<decltype(lim)::value, decltype(rs)::value, EOS_PERFECT_GAS>();
         });
     }
+}
+
+void march1d_exact(const GridDev& g, const StateDev& st0, const StateDev& st1, StepCtl* ctl, const RunParamsDev& rp,
+                 int slot0, int steps, cudaStream_t s)
+{
+    march1d64_launch_t<EOS_PERFECT_GAS>(g, st0, st1, ctl, rp, slot0, steps, s);
 }
 
 void march2d_exact(const GridDev& g, const StateDev& in, const StateDev& out, StepCtl* ctl, const RunParamsDev& rp,

@@ -571,48 +571,39 @@ __device__ __forceinline__ double sound(const Eos& e, double rho, double P)
 }
 
 // What the health check and the CFL need of a new state: the internal energy
-// (main.cpp:397-425), |u_d| and the sound speed (time_step.hpp:55-77).
+// (main.cpp:397-425), the primitives and the sound speed (time_step.hpp:55-77).
 template <int ND>
-static __device__ __noinline__ void state_speeds_slow(Eos e, const double* q, double* out)
+static __device__ __noinline__ void state_prims_slow(Eos e, const double* q, double* out)
 {
-    double pr[ND + 2];
     out[0] = q[1 + ND] - plain::ek_cons<ND>(q);
-    plain::to_prim<ND>(e, q, pr);
-    out[1] = plain_sound(e, pr[0], pr[1 + ND]);
-    for (int d = 0; d < ND; ++d) {
-        out[2 + d] = fabs(pr[1 + d]);
-    }
+    plain::to_prim<ND>(e, q, out + 2);
+    out[1] = plain_sound(e, out[2], out[3 + ND]);
 }
 template <int ND>
-__device__ __forceinline__ void state_speeds(const Eos& e, const double* q, double& evol, double& snd, double* absu)
+__device__ __forceinline__ void state_prims(const Eos& e, const double* q, double& evol, double& snd, double* p)
 {
     bool slow = e.kind == EOS_RAD_GAS;
     if (e.kind != EOS_RAD_GAS) {
-        double pr[ND + 2];
         q64::Den r, k;
         q64::Range S(e.consts_ok), Z;
-        prim_core<ND>(e, q, pr, r, k, evol, S, Z);
-        snd = q64::root(q64::quo(e.gamma * pr[1 + ND], r));
-#pragma unroll
-        for (int d = 0; d < ND; ++d) {
-            absu[d] = fabs(pr[1 + d]);
-        }
+        prim_core<ND>(e, q, p, r, k, evol, S, Z);
+        snd = q64::root(q64::quo(e.gamma * p[1 + ND], r));
         if (!(S.ok() && Z.ok())) {
             slow = !(S.ok() && prim_zeros<ND>(e, q));
         }
     }
     if (slow) {
-        double qt[ND + 2], ot[ND + 2];
+        double qt[ND + 2], ot[ND + 4];
 #pragma unroll
         for (int v = 0; v < ND + 2; ++v) {
             qt[v] = q[v];
         }
-        state_speeds_slow<ND>(e, qt, ot);
+        state_prims_slow<ND>(e, qt, ot);
         evol = ot[0];
         snd = ot[1];
 #pragma unroll
-        for (int d = 0; d < ND; ++d) {
-            absu[d] = ot[2 + d];
+        for (int v = 0; v < ND + 2; ++v) {
+            p[v] = ot[2 + v];
         }
     }
 }
