@@ -105,8 +105,6 @@ struct hcl_handle {
     double *dcot = nullptr, *dsin1 = nullptr, *dsinxc1 = nullptr;
     double* dshell_dv = nullptr;  // InternalMassGravity: the shells' volumes
     double* grav_shell = nullptr; // InternalMassGravity: shell means of rho (nx0 + ng)
-    // stage-path scratch (MUSCLHancockHydroReconstruction's P_rec/u_rec, fx_rec_old)
-    double *u_rec = nullptr, *P_rec = nullptr, *fx_rec_old = nullptr;
     // reductions
     unsigned long long* red_bits = nullptr;
     int* red_flag = nullptr;
@@ -196,9 +194,6 @@ void free_handle(hcl_handle* h)
     cudaFree(h->dcot);
     cudaFree(h->dsin1);
     cudaFree(h->dsinxc1);
-    cudaFree(h->u_rec);
-    cudaFree(h->P_rec);
-    cudaFree(h->fx_rec_old);
     cudaFree(h->red_bits);
     cudaFree(h->red_flag);
     cudaFree(h->red_partials);
@@ -993,26 +988,8 @@ int hcl_hydro_reconstruction(hcl_handle* h, int ng_eff, double dt, const double*
     if (h->g.nfx > 0 && (!fx || !fx_rec)) {
         return fail(HCL_ERR_ARGUMENT, "nfx > 0 needs fx and fx_rec");
     }
-    const int nd = h->g.ndim;
-    const size_t N = (size_t)h->g.N;
-    int rc;
-    if (!u_rec) {
-        if (!h->u_rec && (rc = dalloc(&h->u_rec, N * 2 * nd * nd))) {
-            return rc;
-        }
-        u_rec = h->u_rec;
-    }
-    if (!P_rec) {
-        if (!h->P_rec && (rc = dalloc(&h->P_rec, N * 2 * nd))) {
-            return rc;
-        }
-        P_rec = h->P_rec;
-    }
-    if (h->g.nfx > 0 && !h->fx_rec_old && (rc = dalloc(&h->fx_rec_old, N * 2 * nd * h->g.nfx))) {
-        return rc;
-    }
     hcl::stage::hydro_reconstruction(h->g, ng_eff, dt, rho, u, P, fx, rho_rec, rhou_rec, E_rec, fx_rec, u_rec, P_rec,
-                                     h->fx_rec_old, pick(h, stream));
+                                     pick(h, stream));
     HCL_LAUNCH_CHECK();
     return HCL_OK;
 }
@@ -2811,40 +2788,12 @@ int hcl_ensemble_adjoint(hcl_ensemble* e, const double* const* lam_final, double
 
 } // extern "C"
 
-// ---- hydro reconstruction with fixed scratch (no allocation) ------------------------
-// hcl_hydro_reconstruction_noalloc keeps the scratch of one call (u_rec, P_rec and
-// fx_rec_old of MUSCLHancockHydroReconstruction) in one fixed device array per
-// device instead of the handle's lazily allocated buffers.
+// ---- hydro reconstruction for callers whose loop must not allocate -----------------
 namespace {
 
-constexpr size_t kNoAllocScratchDoubles = size_t(1) << 22; // 32 MiB
-__device__ __align__(256) double g_noalloc_scratch[kNoAllocScratchDoubles];
-
-constexpr int kNoAllocMaxDevices = 64;
-std::mutex g_noalloc_mutex;
-double* g_noalloc_base[kNoAllocMaxDevices] = {};
-
-// Device address of this device's copy of the array, looked up on the first
-// call on each device (the caller has made that device current) and kept for
-// the process: a cudaDeviceReset of that device after the first call leaves
-// the kept address stale, which the header states.
-int noalloc_scratch(int dev, double** out)
-{
-    if (dev < 0 || dev >= kNoAllocMaxDevices) {
-        return fail(HCL_ERR_ARGUMENT, "device %d out of range for the fixed scratch", dev);
-    }
-    std::lock_guard<std::mutex> lock(g_noalloc_mutex);
-    if (!g_noalloc_base[dev]) {
-        void* p = nullptr;
-        const cudaError_t err = cudaGetSymbolAddress(&p, g_noalloc_scratch);
-        if (err != cudaSuccess || !p) {
-            return fail(HCL_ERR_CUDA, "cudaGetSymbolAddress of the fixed scratch failed: %s", cudaGetErrorString(err));
-        }
-        g_noalloc_base[dev] = static_cast<double*>(p);
-    }
-    *out = g_noalloc_base[dev];
-    return HCL_OK;
-}
+// The entry point's documented size limit: the scratch of the reference's
+// MUSCLHancockHydroReconstruction (u_rec, P_rec, fx_rec_old) in 32 MiB.
+constexpr size_t kNoAllocScratchDoubles = size_t(1) << 22;
 
 } // namespace
 
@@ -2879,15 +2828,12 @@ int hcl_hydro_reconstruction_noalloc(hcl_handle* h, int ng_eff, double dt, const
     if (prev != h->cfg.device) {
         HCL_CUDA(cudaSetDevice(h->cfg.device));
     }
-    double* base = nullptr;
-    int rc = noalloc_scratch(h->cfg.device, &base);
-    if (rc == HCL_OK) {
-        hcl::stage::hydro_reconstruction(h->g, ng_eff, dt, rho, u, P, fx, rho_rec, rhou_rec, E_rec, fx_rec, base,
-                                         base + n_u, h->g.nfx > 0 ? base + n_u + n_p : nullptr, pick(h, stream));
-        const cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) {
-            rc = fail(HCL_ERR_CUDA, "kernel launch failed: %s", cudaGetErrorString(e));
-        }
+    int rc = HCL_OK;
+    hcl::stage::hydro_reconstruction(h->g, ng_eff, dt, rho, u, P, fx, rho_rec, rhou_rec, E_rec, fx_rec, nullptr, nullptr,
+                                     pick(h, stream));
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) {
+        rc = fail(HCL_ERR_CUDA, "kernel launch failed: %s", cudaGetErrorString(e));
     }
     if (prev != h->cfg.device) {
         cudaSetDevice(prev);

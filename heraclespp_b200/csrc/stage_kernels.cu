@@ -161,205 +161,221 @@ __global__ void k_face_recon(GridDev g, Box bx, const double* __restrict__ var, 
     }
 }
 
-// hydro_reconstruction.hpp:111-126: face primitives -> face conservatives
+// The whole hydro reconstruction of one cell in one pass: limited face values
+// (hydro_reconstruction.hpp:99-109), face conservatives (:111-126), the Hancock
+// predictor (extrapolation_reconstruction.hpp:90-325) and the passive scalars
+// (:315-339).  u_rec and P_rec receive the face velocities and pressures when
+// not null; fx_rec works in place.
+//
+// Run as the reference's separate kernels (a reconstruction per variable, the
+// conversion, the predictor) the face arrays crossed memory five times; here
+// they are written once, 35 planes in and out for 3-D (41 us for 120 x 100 x 70
+// at the copy rate).  The face states of all but the last dimension wait for
+// the increments of the others in shared memory, where registers would spill.
 template <int ND>
-__global__ void k_faces_prim_to_cons(GridDev g, Box bx, const double* __restrict__ rho_rec,
-                                     const double* __restrict__ u_rec, const double* __restrict__ P_rec,
-                                     double* __restrict__ rhou_rec, double* __restrict__ E_rec)
+__global__ void __launch_bounds__(kThreads, kHeavyMinBlocks)
+k_hydro_reconstruction(GridDev g, Box bx, double dt, const double* __restrict__ rho, const double* __restrict__ u,
+                       const double* __restrict__ P, const double* __restrict__ fx, double* __restrict__ rho_rec,
+                       double* __restrict__ rhou_rec, double* __restrict__ E_rec, double* __restrict__ fx_rec,
+                       double* __restrict__ u_rec, double* __restrict__ P_rec)
 {
-    const exact::Eos eos = exact::eos_of(g);
-    const int64_t S5 = 2 * g.N;
-    const int64_t S6 = 2 * g.N * ND;
-    for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < bx.count;
-         idx += (int64_t)gridDim.x * blockDim.x) {
-        int i, j, k;
-        box_ijk(bx, idx, i, j, k);
-        const int64_t c = lidx(g, i, j, k);
-#pragma unroll
-        for (int idim = 0; idim < ND; ++idim) {
-#pragma unroll
-            for (int s = 0; s < 2; ++s) {
-                const int64_t o = c + g.N * s + S5 * idim;
-                double p[ND + 2], q[ND + 2];
-                p[0] = rho_rec[o];
-#pragma unroll
-                for (int r = 0; r < ND; ++r) {
-                    p[1 + r] = u_rec[o + S6 * r];
-                }
-                p[1 + ND] = P_rec[o];
-                exact::to_cons<ND>(eos, p, q);
-#pragma unroll
-                for (int r = 0; r < ND; ++r) {
-                    rhou_rec[o + S6 * r] = q[1 + r];
-                }
-                E_rec[o] = q[1 + ND];
-            }
-        }
-    }
-}
-
-// extrapolation_reconstruction.hpp:90-325 "Hancock_extrapolation"
-template <int ND>
-__global__ void __launch_bounds__(kThreads, kHeavyMinBlocks) k_hancock(GridDev g, Box bx, double dt, const double* __restrict__ u_rec,
-                          const double* __restrict__ P_rec, double* __restrict__ rho_rec, double* __restrict__ rhou_rec,
-                          double* __restrict__ E_rec, double* __restrict__ fx_rec, const double* __restrict__ fx_rec_old)
-{
+    constexpr int NV = ND + 2;
+    __shared__ double s_face[ND > 1 ? 2 * (ND - 1) : 1][NV][kThreads];
     const exact::Eos eos = exact::eos_of(g);
     const int64_t N = g.N;
     const int64_t S5 = 2 * N;
     const int64_t S6 = 2 * N * ND;
-    const int nfx = g.nfx;
     const bool sph = g.geom == GEOM_SPHERICAL;
+    const int tid = threadIdx.x;
     for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < bx.count;
          idx += (int64_t)gridDim.x * blockDim.x) {
-        int i, j, k;
-        box_ijk(bx, idx, i, j, k);
-        const int64_t c = lidx(g, i, j, k);
-        double rho_old[2][ND];
-        double rhou_old[2][ND][ND];
+        int ijk[3];
+        box_ijk(bx, idx, ijk[0], ijk[1], ijk[2]);
+        const int64_t c = lidx(g, ijk[0], ijk[1], ijk[2]);
+        const int64_t step[3] = {1, g.n[0], (int64_t)g.n[0] * g.n[1]};
+        const double dtodv = dt / g.dv[c];
+        double last[2][NV];     // faces of the last dimension
+        double inc[ND][NV];     // dt/dv (F_L S_L - F_R S_R) per dimension
+        double src[2][5];       // geometric terms of dimensions 0 and 1
+        double mass[2][ND];
 #pragma unroll
-        for (int idim = 0; idim < ND; ++idim) {
-            rho_old[0][idim] = rho_rec[c + S5 * idim];
-            rho_old[1][idim] = rho_rec[c + N + S5 * idim];
+        for (int d = 0; d < ND; ++d) {
+            const double dl = g.dx[d][ijk[d]];
+            const double dl_m = g.dx[d][ijk[d] - 1];
+            const double dl_p = g.dx[d][ijk[d] + 1];
+            double m[NV], v0[NV], p[NV], f[2][NV], U[2][NV], F[2][NV];
+            const int64_t cm = c - step[d], cp = c + step[d];
+            m[0] = rho[cm];
+            v0[0] = rho[c];
+            p[0] = rho[cp];
 #pragma unroll
             for (int r = 0; r < ND; ++r) {
-                rhou_old[0][idim][r] = rhou_rec[c + S5 * idim + S6 * r];
-                rhou_old[1][idim][r] = rhou_rec[c + N + S5 * idim + S6 * r];
+                m[1 + r] = u[cm + N * r];
+                v0[1 + r] = u[c + N * r];
+                p[1 + r] = u[cp + N * r];
             }
-            for (int f = 0; f < nfx; ++f) {
-                const int64_t of = c + S5 * idim + S6 * f;
-                fx_rec[of] *= rho_rec[c + S5 * idim];
-                fx_rec[of + N] *= rho_rec[c + N + S5 * idim];
+            m[1 + ND] = P[cm];
+            v0[1 + ND] = P[c];
+            p[1 + ND] = P[cp];
+            exact::faces<NV>(EOS_PERFECT_GAS, g.limiter, false, m, v0, p, dl_m, dl, dl_p, f[0], f[1]);
+            const double dsc = g.ds[c + N * d];
+            const double dsp = g.ds[cp + N * d];
+#pragma unroll
+            for (int sd = 0; sd < 2; ++sd) {
+                exact::to_cons_flux<ND>(eos, f[sd], d, U[sd], F[sd]);
+                mass[sd][d] = F[sd][0];
+                const int64_t o = c + N * sd + S5 * d;
+                if (u_rec) {
+#pragma unroll
+                    for (int r = 0; r < ND; ++r) {
+                        u_rec[o + S6 * r] = f[sd][1 + r];
+                    }
+                }
+                if (P_rec) {
+                    P_rec[o] = f[sd][1 + ND];
+                }
+#pragma unroll
+                for (int v = 0; v < NV; ++v) {
+                    if (d == ND - 1) {
+                        last[sd][v] = U[sd][v];
+                    } else {
+                        s_face[2 * d + sd][v][tid] = U[sd][v];
+                    }
+                }
+            }
+#pragma unroll
+            for (int v = 0; v < NV; ++v) {
+                inc[d][v] = dtodv * ((F[0][v] * dsc) - (F[1][v] * dsp));
+            }
+            if (sph) { // :145-303
+                const double *pL = f[0], *pR = f[1];
+                if (d == 0) {
+                    src[0][0] = exact::src_grad_pres(dtodv, pL[1 + ND], pR[1 + ND], dsc, dsp);
+                    if constexpr (ND >= 2) {
+                        src[0][1] = exact::src_grad_u_r(dtodv, pL[0], pR[0], pL[2], pR[2], dsc, dsp);
+                        src[0][2] = exact::src_grad_u_idir_r(dtodv, g.x[0][ijk[0]], g.x[0][ijk[0] + 1], pL[0], pR[0],
+                                                             pL[1], pR[1], pL[2], pR[2], dsc, dsp);
+                    }
+                    if constexpr (ND == 3) {
+                        src[0][3] = exact::src_grad_u_r(dtodv, pL[0], pR[0], pL[3], pR[3], dsc, dsp);
+                        src[0][4] = exact::src_grad_u_idir_r(dtodv, g.x[0][ijk[0]], g.x[0][ijk[0] + 1], pL[0], pR[0],
+                                                             pL[1], pR[1], pL[3], pR[3], dsc, dsp);
+                    }
+                }
+                if (d == 1) {
+                    src[1][0] = exact::src_grad_pres(dtodv, pL[1 + ND], pR[1 + ND], dsc, dsp);
+                    if constexpr (ND == 3) {
+                        src[1][1] = exact::src_grad_u_th(dtodv, g.cot_mid1[ijk[1]], pL[0], pR[0], pL[3], pR[3], dsc, dsp);
+                        src[1][2] = exact::src_grad_u_phi(dtodv, g.sin1[ijk[1]], g.sin1[ijk[1] + 1], pL[0], pR[0], pL[2],
+                                                          pR[2], pL[3], pR[3], dsc, dsp);
+                    }
+                }
             }
         }
+        double rho_old[2][ND], rho_new[2][ND];
 #pragma unroll
-        for (int idim = 0; idim < ND; ++idim) {
-            const int64_t cp = lidx(g, i + (idim == 0), j + (idim == 1), k + (idim == 2));
-            double pL[ND + 2], pR[ND + 2], fL[ND + 2], fR[ND + 2];
-            pL[0] = rho_old[0][idim];
-            pR[0] = rho_old[1][idim];
+        for (int ip = 0; ip < ND; ++ip) {
 #pragma unroll
-            for (int r = 0; r < ND; ++r) {
-                pL[1 + r] = u_rec[c + S5 * idim + S6 * r];
-                pR[1 + r] = u_rec[c + N + S5 * idim + S6 * r];
-            }
-            pL[1 + ND] = P_rec[c + S5 * idim];
-            pR[1 + ND] = P_rec[c + N + S5 * idim];
-            exact::flux_prim<ND>(eos, pL, idim, fL);
-            exact::flux_prim<ND>(eos, pR, idim, fR);
-            const double dtodv = dt / g.dv[c];
-            const double dsc = g.ds[c + N * idim];
-            const double dsp = g.ds[cp + N * idim];
+            for (int sd = 0; sd < 2; ++sd) {
+                double U[NV];
 #pragma unroll
-            for (int ipos = 0; ipos < ND; ++ipos) {
-                const int64_t o0 = c + S5 * ipos;
-                const int64_t o1 = o0 + N;
-                rho_rec[o0] += dtodv * ((fL[0] * dsc) - (fR[0] * dsp));
-                rho_rec[o1] += dtodv * ((fL[0] * dsc) - (fR[0] * dsp));
+                for (int v = 0; v < NV; ++v) {
+                    U[v] = ip == ND - 1 ? last[sd][v] : s_face[2 * ip + sd][v][tid];
+                }
+                const double old0 = U[0];
+                double mom[ND];
 #pragma unroll
                 for (int r = 0; r < ND; ++r) {
-                    rhou_rec[o0 + S6 * r] += dtodv * ((fL[1 + r] * dsc) - (fR[1 + r] * dsp));
-                    rhou_rec[o1 + S6 * r] += dtodv * ((fL[1 + r] * dsc) - (fR[1 + r] * dsp));
+                    mom[r] = U[1 + r];
                 }
-                E_rec[o0] += dtodv * ((fL[1 + ND] * dsc) - (fR[1 + ND] * dsp));
-                E_rec[o1] += dtodv * ((fL[1 + ND] * dsc) - (fR[1 + ND] * dsp));
-            }
-            if (sph) {
-                // :145-303
-                const double PL = pL[1 + ND], PR = pR[1 + ND];
 #pragma unroll
-                for (int ipos = 0; ipos < ND; ++ipos) {
-                    const int64_t o0 = c + S5 * ipos;
-                    const int64_t o1 = o0 + N;
-                    if (idim == 0) {
-                        const double sp = exact::src_grad_pres(dtodv, PL, PR, dsc, dsp);
-                        rhou_rec[o0 + S6 * idim] += sp;
-                        rhou_rec[o1 + S6 * idim] += sp;
+                for (int d = 0; d < ND; ++d) {
+#pragma unroll
+                    for (int v = 0; v < NV; ++v) {
+                        U[v] += inc[d][v];
+                    }
+                    if (sph && d == 0) {
+                        U[1] += src[0][0];
                         if constexpr (ND >= 2) {
-                            const double sr = exact::src_grad_u_r(dtodv, pL[0], pR[0], pL[2], pR[2], dsc, dsp);
-                            rhou_rec[o0 + S6 * idim] += sr;
-                            rhou_rec[o1 + S6 * idim] += sr;
-                            const double st = exact::src_grad_u_idir_r(dtodv, g.x[0][i], g.x[0][i + 1], pL[0], pR[0],
-                                                                       pL[1], pR[1], pL[2], pR[2], dsc, dsp);
-                            rhou_rec[o0 + S6 * 1] -= st;
-                            rhou_rec[o1 + S6 * 1] -= st;
+                            U[1] += src[0][1];
+                            U[2] -= src[0][2];
                         }
                         if constexpr (ND == 3) {
-                            const double sr = exact::src_grad_u_r(dtodv, pL[0], pR[0], pL[3], pR[3], dsc, dsp);
-                            rhou_rec[o0 + S6 * idim] += sr;
-                            rhou_rec[o1 + S6 * idim] += sr;
-                            const double sf = exact::src_grad_u_idir_r(dtodv, g.x[0][i], g.x[0][i + 1], pL[0], pR[0],
-                                                                       pL[1], pR[1], pL[3], pR[3], dsc, dsp);
-                            rhou_rec[o0 + S6 * 2] -= sf;
-                            rhou_rec[o1 + S6 * 2] -= sf;
+                            U[1] += src[0][3];
+                            U[3] -= src[0][4];
                         }
                     }
-                    if (idim == 1) {
-                        const double sp = exact::src_grad_pres(dtodv, PL, PR, dsc, dsp);
-                        rhou_rec[o0 + S6 * idim] += sp;
-                        rhou_rec[o1 + S6 * idim] += sp;
-                        if constexpr (ND == 3) {
-                            const double sth = exact::src_grad_u_th(dtodv, g.cot_mid1[j], pL[0], pR[0], pL[3], pR[3], dsc, dsp);
-                            rhou_rec[o0 + S6 * idim] += sth;
-                            rhou_rec[o1 + S6 * idim] += sth;
-                            const double sph2 = exact::src_grad_u_phi(dtodv, g.sin1[j], g.sin1[j + 1], pL[0], pR[0],
-                                                                      pL[2], pR[2], pL[3], pR[3], dsc, dsp);
-                            rhou_rec[o0 + S6 * 2] -= sph2;
-                            rhou_rec[o1 + S6 * 2] -= sph2;
+                    if constexpr (ND >= 2) {
+                        if (sph && d == 1) {
+                            U[2] += src[1][0];
+                            if constexpr (ND == 3) {
+                                U[2] += src[1][1];
+                                U[3] -= src[1][2];
+                            }
                         }
                     }
+                    const double gd = gravity_at(g, ijk[0], d); // :306-312
+                    U[1 + d] += dt * gd * old0;
+                    U[1 + ND] += dt * gd * mom[d];
                 }
-            }
-            // gravity :306-312
-            const double gd = gravity_at(g, i, idim);
+                rho_old[sd][ip] = old0;
+                rho_new[sd][ip] = U[0];
+                const int64_t o = c + N * sd + S5 * ip;
+                rho_rec[o] = U[0];
 #pragma unroll
-            for (int ipos = 0; ipos < ND; ++ipos) {
-                const int64_t o0 = c + S5 * ipos;
-                const int64_t o1 = o0 + N;
-                rhou_rec[o0 + S6 * idim] += dt * gd * rho_old[0][ipos];
-                rhou_rec[o1 + S6 * idim] += dt * gd * rho_old[1][ipos];
-                E_rec[o0] += dt * gd * rhou_old[0][ipos][idim];
-                E_rec[o1] += dt * gd * rhou_old[1][ipos][idim];
+                for (int r = 0; r < ND; ++r) {
+                    rhou_rec[o + S6 * r] = U[1 + r];
+                }
+                E_rec[o] = U[1 + ND];
             }
-            // passive scalars :315-337
-            for (int f = 0; f < nfx; ++f) {
-                const int64_t off = S6 * f;
-                const double ffL = fx_rec_old[c + S5 * idim + off] * fL[0];
-                const double ffR = fx_rec_old[c + N + S5 * idim + off] * fR[0];
+        }
+        for (int f = 0; f < g.nfx; ++f) {
+            const double* x = fx + N * f;
+            double xf[2][ND];
 #pragma unroll
-                for (int ipos = 0; ipos < ND; ++ipos) {
-                    const int64_t o0 = c + S5 * ipos + off;
-                    fx_rec[o0] += dtodv * ((ffL * dsc) - (ffR * dsp));
-                    fx_rec[o0 + N] += dtodv * ((ffL * dsc) - (ffR * dsp));
+            for (int d = 0; d < ND; ++d) {
+                const double m = x[c - step[d]], v0 = x[c], p = x[c + step[d]];
+                exact::faces<1>(EOS_PERFECT_GAS, g.limiter, false, &m, &v0, &p, g.dx[d][ijk[d] - 1], g.dx[d][ijk[d]],
+                                g.dx[d][ijk[d] + 1], &xf[0][d], &xf[1][d]);
+            }
+#pragma unroll
+            for (int ip = 0; ip < ND; ++ip) {
+#pragma unroll
+                for (int sd = 0; sd < 2; ++sd) {
+                    double v = xf[sd][ip] * rho_old[sd][ip];
+#pragma unroll
+                    for (int d = 0; d < ND; ++d) {
+                        const double dsc = g.ds[c + N * d];
+                        const double dsp = g.ds[c + step[d] + N * d];
+                        v += dtodv * (((xf[0][d] * mass[0][d]) * dsc) - ((xf[1][d] * mass[1][d]) * dsp));
+                    }
+                    fx_rec[c + N * sd + S5 * ip + S6 * f] = v / rho_new[sd][ip];
                 }
             }
         }
     }
 }
 
-// extrapolation_reconstruction.hpp:329-339 "passive_scalar_extrapolation"
+// godunov_scheme.hpp:110-292 "Riemann_based_Godunov_scheme" on tiles: each
+// face's Riemann problem is solved once (the reference solves it from both
+// sides), its flux kept in shared memory, then every cell of the tile updates.
+// 32 x 4 x 2 cells in 3-D: 968 faces instead of 1536 solves.  A warp takes rows
+// of 32 faces of one dimension; the tile's last x-faces form one more row.
 template <int ND>
-__global__ void k_passive_extrap(GridDev g, Box bx, const double* __restrict__ rho_rec, double* __restrict__ fx_rec)
-{
-    const int64_t N = g.N;
-    const int64_t S5 = 2 * N;
-    const int64_t S6 = 2 * N * ND;
-    for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < bx.count;
-         idx += (int64_t)gridDim.x * blockDim.x) {
-        int i, j, k;
-        box_ijk(bx, idx, i, j, k);
-        const int64_t c = lidx(g, i, j, k);
-        for (int idim = 0; idim < ND; ++idim) {
-            for (int f = 0; f < g.nfx; ++f) {
-                const int64_t o = c + S5 * idim + S6 * f;
-                fx_rec[o] /= rho_rec[c + S5 * idim];
-                fx_rec[o + N] /= rho_rec[c + N + S5 * idim];
-            }
-        }
+struct GodTile {
+    static constexpr int NV = ND + 2;
+    static constexpr int T[3] = {ND == 1 ? kThreads : 32, ND == 1 ? 1 : (ND == 2 ? 8 : 4), ND == 3 ? 2 : 1};
+    static constexpr int NF(int d)
+    {
+        return (T[0] + (d == 0)) * (T[1] + (d == 1)) * (T[2] + (d == 2));
     }
-}
+    static constexpr int off(int d)
+    {
+        return d == 0 ? 0 : (d == 1 ? NF(0) : NF(0) + NF(1));
+    }
+    static constexpr int total = NF(0) + (ND > 1 ? NF(1) : 0) + (ND > 2 ? NF(2) : 0);
+};
 
-// godunov_scheme.hpp:110-292 "Riemann_based_Godunov_scheme"
 template <int ND>
 __global__ void __launch_bounds__(kThreads, kHeavyMinBlocks) k_godunov(GridDev g, Box bx, double dt, const double* __restrict__ rho, const double* __restrict__ rhou,
                           const double* __restrict__ E, const double* __restrict__ fx,
@@ -368,115 +384,175 @@ __global__ void __launch_bounds__(kThreads, kHeavyMinBlocks) k_godunov(GridDev g
                           double* __restrict__ rho_new, double* __restrict__ rhou_new, double* __restrict__ E_new,
                           double* __restrict__ fx_new)
 {
+    using T = GodTile<ND>;
+    constexpr int NV = ND + 2;
+    constexpr int T0 = T::T[0], T1 = T::T[1], T2 = T::T[2];
+    __shared__ double s_flux[NV][T::total];
     const exact::Eos eos = exact::eos_of(g);
     const int64_t N = g.N;
     const int64_t S5 = 2 * N;
     const int64_t S6 = 2 * N * ND;
     const bool sph = g.geom == GEOM_SPHERICAL;
-    for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < bx.count;
-         idx += (int64_t)gridDim.x * blockDim.x) {
-        int i, j, k;
-        box_ijk(bx, idx, i, j, k);
+    const int64_t step[3] = {1, g.n[0], (int64_t)g.n[0] * g.n[1]};
+    const int tid = threadIdx.x;
+    const int lane = tid & 31;
+    const int nt0 = (bx.w[0] + T0 - 1) / T0;
+    const int nt1 = (bx.w[1] + T1 - 1) / T1;
+    const int org[3] = {bx.b[0] + (int)(blockIdx.x % nt0) * T0, bx.b[1] + (int)(blockIdx.x / nt0 % nt1) * T1,
+                        bx.b[2] + (int)(blockIdx.x / nt0 / nt1) * T2};
+    const int end[3] = {bx.b[0] + bx.w[0], bx.b[1] + bx.w[1], bx.b[2] + bx.w[2]};
+
+    // face f = (a0, a1, a2) of dimension d: between the cells at org + a - 1_d
+    // and org + a
+    auto solve = [&](auto dc, int a0, int a1, int a2) {
+        constexpr int d = decltype(dc)::value;
+        const int i = org[0] + a0, j = org[1] + a1, k = org[2] + a2;
+        if (i >= end[0] + (d == 0) || j >= end[1] + (d == 1) || k >= end[2] + (d == 2)) {
+            return;
+        }
         const int64_t c = lidx(g, i, j, k);
-        double rn = rho[c];
-        double En = E[c];
-        double mn[ND];
+        const int64_t oL = c - step[d] + N + S5 * d; // right state of the left cell
+        const int64_t oR = c + S5 * d;
+        double cL[NV], cR[NV], F[NV];
+        cL[0] = rho_rec[oL];
+        cR[0] = rho_rec[oR];
 #pragma unroll
-        for (int d = 0; d < ND; ++d) {
-            mn[d] = rhou[c + N * d];
+        for (int r = 0; r < ND; ++r) {
+            cL[1 + r] = rhou_rec[oL + S6 * r];
+            cR[1 + r] = rhou_rec[oR + S6 * r];
         }
-        for (int f = 0; f < g.nfx; ++f) {
-            fx_new[c + N * f] = fx[c + N * f] * rho[c];
+        cL[1 + ND] = E_rec[oL];
+        cR[1 + ND] = E_rec[oR];
+        exact::riemann<ND>(eos, g.riemann, cL, cR, d, F);
+        const int f = T::off(d) + a0 + (T0 + (d == 0)) * (a1 + (T1 + (d == 1)) * a2);
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            s_flux[v][f] = F[v];
         }
-#pragma unroll
-        for (int idim = 0; idim < ND; ++idim) {
-            const int64_t cm = lidx(g, i - (idim == 0), j - (idim == 1), k - (idim == 2));
-            const int64_t cp = lidx(g, i + (idim == 0), j + (idim == 1), k + (idim == 2));
-            double mR[ND + 2], vL[ND + 2], vR[ND + 2], pLn[ND + 2], FL[ND + 2], FR[ND + 2];
-            mR[0] = rho_rec[cm + N + S5 * idim];
-            vL[0] = rho_rec[c + S5 * idim];
-            vR[0] = rho_rec[c + N + S5 * idim];
-            pLn[0] = rho_rec[cp + S5 * idim];
-#pragma unroll
-            for (int r = 0; r < ND; ++r) {
-                mR[1 + r] = rhou_rec[cm + N + S5 * idim + S6 * r];
-                vL[1 + r] = rhou_rec[c + S5 * idim + S6 * r];
-                vR[1 + r] = rhou_rec[c + N + S5 * idim + S6 * r];
-                pLn[1 + r] = rhou_rec[cp + S5 * idim + S6 * r];
+    };
+    constexpr int B0 = T0 / 32;          // row blocks along x
+    constexpr int R0 = B0 * T1 * T2;     // rows of x-faces
+    constexpr int RX = (T1 * T2 + 31) / 32; // the last x-faces
+    constexpr int R1 = ND > 1 ? B0 * (T1 + 1) * T2 : 0;
+    constexpr int R2 = ND > 2 ? B0 * T1 * (T2 + 1) : 0;
+#pragma unroll 1
+    for (int t = tid >> 5; t < R0 + RX + R1 + R2; t += kThreads / 32) {
+        if (t < R0) {
+            const int q = t / B0;
+            solve(std::integral_constant<int, 0>{}, (t % B0) * 32 + lane, q % T1, q / T1);
+        } else if (t < R0 + RX) {
+            const int q = (t - R0) * 32 + lane;
+            if (q < T1 * T2) {
+                solve(std::integral_constant<int, 0>{}, T0, q % T1, q / T1);
             }
-            mR[1 + ND] = E_rec[cm + N + S5 * idim];
-            vL[1 + ND] = E_rec[c + S5 * idim];
-            vR[1 + ND] = E_rec[c + N + S5 * idim];
-            pLn[1 + ND] = E_rec[cp + S5 * idim];
-            exact::riemann<ND>(eos, g.riemann, mR, vL, idim, FL);
-            exact::riemann<ND>(eos, g.riemann, vR, pLn, idim, FR);
-            const double dtodv = dt / g.dv[c];
-            const double dsc = g.ds[c + N * idim];
-            const double dsp = g.ds[cp + N * idim];
-            rn += dtodv * ((FL[0] * dsc) - (FR[0] * dsp));
-#pragma unroll
-            for (int r = 0; r < ND; ++r) {
-                mn[r] += dtodv * ((FL[1 + r] * dsc) - (FR[1 + r] * dsp));
+        } else if (t < R0 + RX + R1) {
+            if constexpr (ND > 1) {
+                const int r = t - R0 - RX, q = r / B0;
+                solve(std::integral_constant<int, 1>{}, (r % B0) * 32 + lane, q % (T1 + 1), q / (T1 + 1));
             }
-            En += dtodv * ((FL[1 + ND] * dsc) - (FR[1 + ND] * dsp));
-            if (sph) {
-                // :165-256
-                double pl[ND + 2], pr[ND + 2];
-                exact::to_prim<ND>(eos, vL, pl);
-                exact::to_prim<ND>(eos, vR, pr);
-                if (idim == 0) {
-                    mn[0] += exact::src_grad_pres(dtodv, pl[1 + ND], pr[1 + ND], dsc, dsp);
-                    if constexpr (ND >= 2) {
-                        mn[0] += exact::src_grad_u_r(dtodv, pl[0], pr[0], pl[2], pr[2], dsc, dsp);
-                        mn[1] -= exact::src_grad_u_idir_r(dtodv, g.x[0][i], g.x[0][i + 1], pl[0], pr[0], pl[1], pr[1],
-                                                          pl[2], pr[2], dsc, dsp);
-                    }
-                    if constexpr (ND == 3) {
-                        mn[0] += exact::src_grad_u_r(dtodv, pl[0], pr[0], pl[3], pr[3], dsc, dsp);
-                        mn[2] -= exact::src_grad_u_idir_r(dtodv, g.x[0][i], g.x[0][i + 1], pl[0], pr[0], pl[1], pr[1],
-                                                          pl[3], pr[3], dsc, dsp);
-                    }
-                }
-                if constexpr (ND >= 2) {
-                    if (idim == 1) {
-                        mn[1] += exact::src_grad_pres(dtodv, pl[1 + ND], pr[1 + ND], dsc, dsp);
-                        if constexpr (ND == 3) {
-                            mn[1] += exact::src_grad_u_th(dtodv, g.cot_mid1[j], pl[0], pr[0], pl[3], pr[3], dsc, dsp);
-                            mn[2] -= exact::src_grad_u_phi(dtodv, g.sin1[j], g.sin1[j + 1], pl[0], pr[0], pl[2], pr[2],
-                                                           pl[3], pr[3], dsc, dsp);
-                        }
-                    }
-                }
-            }
-            // gravity :258-260
-            const double gd = gravity_at(g, i, idim);
-            mn[idim] += dt * gd * rho[c];
-            En += dt * gd * rhou[c + N * idim];
-            // passive scalars :262-290
-            for (int f = 0; f < g.nfx; ++f) {
-                const int64_t off = S6 * f;
-                int64_t iL = cm, iR = c;
-                int64_t sL = 1, sR = 1;
-                if (FL[0] < 0) {
-                    iL = c;
-                    sL = 0;
-                }
-                if (FR[0] < 0) {
-                    iR = cp;
-                    sR = 0;
-                }
-                const double ffL = fx_rec[iL + N * sL + S5 * idim + off] * FL[0];
-                const double ffR = fx_rec[iR + N * sR + S5 * idim + off] * FR[0];
-                fx_new[c + N * f] += dtodv * ((ffL * dsc) - (ffR * dsp));
+        } else {
+            if constexpr (ND > 2) {
+                const int r = t - R0 - RX - R1, q = r / B0;
+                solve(std::integral_constant<int, 2>{}, (r % B0) * 32 + lane, q % T1, q / T1);
             }
         }
-        rho_new[c] = rn;
-#pragma unroll
-        for (int d = 0; d < ND; ++d) {
-            rhou_new[c + N * d] = mn[d];
-        }
-        E_new[c] = En;
     }
+    __syncthreads();
+
+    const int x[3] = {tid % T0, tid / T0 % T1, tid / T0 / T1};
+    const int i = org[0] + x[0], j = org[1] + x[1], k = org[2] + x[2];
+    if (i >= end[0] || j >= end[1] || k >= end[2]) {
+        return;
+    }
+    const int64_t c = lidx(g, i, j, k);
+    const double r_old = rho[c];
+    double rn = r_old;
+    double En = E[c];
+    double mo[ND], mn[ND];
+#pragma unroll
+    for (int d = 0; d < ND; ++d) {
+        mo[d] = mn[d] = rhou[c + N * d];
+    }
+    for (int f = 0; f < g.nfx; ++f) {
+        fx_new[c + N * f] = fx[c + N * f] * r_old;
+    }
+    const double dtodv = dt / g.dv[c];
+#pragma unroll
+    for (int d = 0; d < ND; ++d) {
+        const int64_t cm = c - step[d], cp = c + step[d];
+        const int fL = T::off(d) + x[0] + (T0 + (d == 0)) * (x[1] + (T1 + (d == 1)) * x[2]);
+        const int fR = fL + (d == 0 ? 1 : (d == 1 ? T0 : T0 * T1));
+        double FL[NV], FR[NV];
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            FL[v] = s_flux[v][fL];
+            FR[v] = s_flux[v][fR];
+        }
+        const double dsc = g.ds[c + N * d];
+        const double dsp = g.ds[cp + N * d];
+        rn += dtodv * ((FL[0] * dsc) - (FR[0] * dsp));
+#pragma unroll
+        for (int r = 0; r < ND; ++r) {
+            mn[r] += dtodv * ((FL[1 + r] * dsc) - (FR[1 + r] * dsp));
+        }
+        En += dtodv * ((FL[1 + ND] * dsc) - (FR[1 + ND] * dsp));
+        if (sph && d < 2) {
+            // :165-256, from the cell's own face states
+            double vL[NV], vR[NV], pl[NV], pr[NV];
+            const int64_t o = c + S5 * d;
+            vL[0] = rho_rec[o];
+            vR[0] = rho_rec[o + N];
+#pragma unroll
+            for (int r = 0; r < ND; ++r) {
+                vL[1 + r] = rhou_rec[o + S6 * r];
+                vR[1 + r] = rhou_rec[o + N + S6 * r];
+            }
+            vL[1 + ND] = E_rec[o];
+            vR[1 + ND] = E_rec[o + N];
+            exact::to_prim<ND>(eos, vL, pl);
+            exact::to_prim<ND>(eos, vR, pr);
+            if (d == 0) {
+                mn[0] += exact::src_grad_pres(dtodv, pl[1 + ND], pr[1 + ND], dsc, dsp);
+                if constexpr (ND >= 2) {
+                    mn[0] += exact::src_grad_u_r(dtodv, pl[0], pr[0], pl[2], pr[2], dsc, dsp);
+                    mn[1] -= exact::src_grad_u_idir_r(dtodv, g.x[0][i], g.x[0][i + 1], pl[0], pr[0], pl[1], pr[1],
+                                                      pl[2], pr[2], dsc, dsp);
+                }
+                if constexpr (ND == 3) {
+                    mn[0] += exact::src_grad_u_r(dtodv, pl[0], pr[0], pl[3], pr[3], dsc, dsp);
+                    mn[2] -= exact::src_grad_u_idir_r(dtodv, g.x[0][i], g.x[0][i + 1], pl[0], pr[0], pl[1], pr[1],
+                                                      pl[3], pr[3], dsc, dsp);
+                }
+            }
+            if constexpr (ND >= 2) {
+                if (d == 1) {
+                    mn[1] += exact::src_grad_pres(dtodv, pl[1 + ND], pr[1 + ND], dsc, dsp);
+                    if constexpr (ND == 3) {
+                        mn[1] += exact::src_grad_u_th(dtodv, g.cot_mid1[j], pl[0], pr[0], pl[3], pr[3], dsc, dsp);
+                        mn[2] -= exact::src_grad_u_phi(dtodv, g.sin1[j], g.sin1[j + 1], pl[0], pr[0], pl[2], pr[2],
+                                                       pl[3], pr[3], dsc, dsp);
+                    }
+                }
+            }
+        }
+        // gravity :258-260
+        const double gd = gravity_at(g, i, d);
+        mn[d] += dt * gd * r_old;
+        En += dt * gd * mo[d];
+        // passive scalars :262-290
+        for (int f = 0; f < g.nfx; ++f) {
+            const int64_t off = S6 * f + S5 * d;
+            const double ffL = fx_rec[(FL[0] < 0 ? c : cm + N) + off] * FL[0];
+            const double ffR = fx_rec[(FR[0] < 0 ? cp : c + N) + off] * FR[0];
+            fx_new[c + N * f] += dtodv * ((ffL * dsc) - (ffR * dsp));
+        }
+    }
+    rho_new[c] = rn;
+#pragma unroll
+    for (int d = 0; d < ND; ++d) {
+        rhou_new[c + N * d] = mn[d];
+    }
+    E_new[c] = En;
 }
 
 // pressure_fix.hpp:19-172: where the old internal energy is below eps times
@@ -947,38 +1023,15 @@ void face_reconstruction(const GridDev& g, int ng_eff, const double* var, double
 
 void hydro_reconstruction(const GridDev& g, int ng_eff, double dt, const double* rho, const double* u,
                           const double* P, const double* fx, double* rho_rec, double* rhou_rec, double* E_rec,
-                          double* fx_rec, double* u_rec, double* P_rec, double* fx_rec_old, cudaStream_t s)
+                          double* fx_rec, double* u_rec, double* P_rec, cudaStream_t s)
 {
-    const int nd = g.ndim;
-    const int64_t N = g.N;
-    // hydro_reconstruction.hpp:99-109
-    face_reconstruction(g, ng_eff, rho, rho_rec, s);
-    for (int d = 0; d < nd; ++d) {
-        face_reconstruction(g, ng_eff, u + N * d, u_rec + 2 * N * nd * d, s);
-    }
-    face_reconstruction(g, ng_eff, P, P_rec, s);
-    for (int f = 0; f < g.nfx; ++f) {
-        face_reconstruction(g, ng_eff, fx + N * f, fx_rec + 2 * N * nd * f, s);
-    }
     const Box bx = make_box(g, ng_eff);
-    dispatch_nd(nd, [&](auto ndc) {
+    dispatch_nd(g.ndim, [&](auto ndc) {
         constexpr int ND = decltype(ndc)::value;
-        k_faces_prim_to_cons<ND><<<grid_for(bx.count), kThreads, 0, s>>>(g, bx, rho_rec, u_rec, P_rec, rhou_rec, E_rec);
+        k_hydro_reconstruction<ND><<<grid_for(bx.count), kThreads, 0, s>>>(g, bx, dt, rho, u, P, fx, rho_rec, rhou_rec,
+                                                                           E_rec, fx_rec, u_rec, P_rec);
     });
     ++g_launches;
-    // extrapolation_reconstruction.hpp:87-88
-    if (g.nfx > 0) {
-        cudaMemcpyAsync(fx_rec_old, fx_rec, sizeof(double) * (size_t)(2 * N * nd * g.nfx), cudaMemcpyDeviceToDevice, s);
-    }
-    dispatch_nd(nd, [&](auto ndc) {
-        constexpr int ND = decltype(ndc)::value;
-        k_hancock<ND><<<grid_for(bx.count), kThreads, 0, s>>>(g, bx, dt, u_rec, P_rec, rho_rec, rhou_rec, E_rec, fx_rec,
-                                                              fx_rec_old);
-        if (g.nfx > 0) {
-            k_passive_extrap<ND><<<grid_for(bx.count), kThreads, 0, s>>>(g, bx, rho_rec, fx_rec);
-        }
-    });
-    g_launches += g.nfx > 0 ? 2 : 1;
 }
 
 void godunov(const GridDev& g, int ng_eff, double dt, const double* rho, const double* rhou, const double* E,
@@ -989,7 +1042,10 @@ void godunov(const GridDev& g, int ng_eff, double dt, const double* rho, const d
     const Box bx = make_box(g, ng_eff);
     dispatch_nd(g.ndim, [&](auto ndc) {
         constexpr int ND = decltype(ndc)::value;
-        k_godunov<ND><<<grid_for(bx.count), kThreads, 0, s>>>(g, bx, dt, rho, rhou, E, fx, rho_rec, rhou_rec, E_rec,
+        using T = GodTile<ND>;
+        const int64_t blocks = (int64_t)((bx.w[0] + T::T[0] - 1) / T::T[0]) * ((bx.w[1] + T::T[1] - 1) / T::T[1]) *
+                               ((bx.w[2] + T::T[2] - 1) / T::T[2]);
+        k_godunov<ND><<<(unsigned)blocks, kThreads, 0, s>>>(g, bx, dt, rho, rhou, E, fx, rho_rec, rhou_rec, E_rec,
                                                               fx_rec, rho_new, rhou_new, E_new, fx_new);
     });
     ++g_launches;

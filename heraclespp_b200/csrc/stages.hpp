@@ -27,7 +27,7 @@ void temperature(const GridDev& g, int ng_eff, const double* rho, const double* 
 void face_reconstruction(const GridDev& g, int ng_eff, const double* var, double* var_rec, cudaStream_t s);
 void hydro_reconstruction(const GridDev& g, int ng_eff, double dt, const double* rho, const double* u,
                           const double* P, const double* fx, double* rho_rec, double* rhou_rec, double* E_rec,
-                          double* fx_rec, double* u_rec, double* P_rec, double* fx_rec_old, cudaStream_t s);
+                          double* fx_rec, double* u_rec, double* P_rec, cudaStream_t s);
 void godunov(const GridDev& g, int ng_eff, double dt, const double* rho, const double* rhou, const double* E,
              const double* fx, const double* rho_rec, const double* rhou_rec, const double* E_rec,
              const double* fx_rec, double* rho_new, double* rhou_new, double* E_new, double* fx_new,

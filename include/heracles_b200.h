@@ -158,32 +158,23 @@ int hcl_face_reconstruction(hcl_handle* h, int ng_eff, const double* var, double
 /* IHydroReconstruction::execute (hydro/hydro_reconstruction.hpp:46-58,85-129)
  * including HancockExtrapolationReconstruction (extrapolation_reconstruction.hpp:65-338).
  * dt is the reconstruction time step (the reference passes dt/2, main.cpp:427-439).
- * u_rec/P_rec are the scratch views MUSCLHancockHydroReconstruction owns
- * (hydro_reconstruction.hpp:67-68); pass NULL to use the handle's own.
+ * u_rec/P_rec (the scratch views MUSCLHancockHydroReconstruction owns,
+ * hydro_reconstruction.hpp:67-68) receive the face velocities and pressures;
+ * pass NULL to leave them out: the call needs no scratch.
  * fx/fx_rec may be NULL when nfx == 0. */
 int hcl_hydro_reconstruction(hcl_handle* h, int ng_eff, double dt, const double* rho, const double* u,
                              const double* P, const double* fx, double* rho_rec, double* rhou_rec, double* E_rec,
                              double* fx_rec, double* u_rec, double* P_rec, void* stream);
-/* hcl_hydro_reconstruction with its scratch (u_rec, P_rec, fx_rec_old) in one
- * fixed 32 MiB device array per device (2^22 doubles) instead of buffers the
- * handle allocates on first use: the call itself allocates and frees no
- * device memory.  No counterpart in the reference (its
- * MUSCLHancockHydroReconstruction owns Kokkos views allocated at
- * construction).  For host code whose time loop must not allocate after
- * set-up: an allocation there can synchronise the whole device, and a caller
- * that hands all free device memory to its own pool has none to give.
+/* hcl_hydro_reconstruction without u_rec and P_rec, as an entry point that
+ * promises not to allocate or free device memory (an allocation in a time loop
+ * can synchronise the whole device, and a caller that hands all free device
+ * memory to its own pool has none to give).  No counterpart in the reference
+ * (its MUSCLHancockHydroReconstruction owns Kokkos views allocated at
+ * construction).  Switches to the handle's device for the call.
  * Limit: N * 2*ndim*(ndim + 1 + nfx) <= 2^22 doubles, N the cell count with
- * ghosts (2-D, nfx = 0: N <= 349525; 3-D: N <= 174762); larger grids get
- * HCL_ERR_CONFIG.  The first call on a device looks the array up
- * (cudaGetSymbolAddress) and switches to the handle's device for it; make
- * that first call before any stream capture.  The looked-up address is kept
- * for the life of the process: after a cudaDeviceReset of that device (or an
- * unload and reload of this library's module) it no longer names the array,
- * so do not call this entry point on a device that was reset after its first
- * call.  Nothing in the scratch needs to
- * start at zero (each call writes every entry it reads).  The array is shared
- * by all handles on a device: calls whose work overlaps in time on one device
- * (different streams, threads or handles) race on it; order them. */
+ * ghosts (2-D, nfx = 0: N <= 349525; 3-D: N <= 174762), the size of the
+ * scratch of the reference's separate kernels; larger grids get
+ * HCL_ERR_CONFIG. */
 int hcl_hydro_reconstruction_noalloc(hcl_handle* h, int ng_eff, double dt, const double* rho, const double* u,
                                      const double* P, const double* fx, double* rho_rec, double* rhou_rec,
                                      double* E_rec, double* fx_rec, void* stream);
