@@ -346,7 +346,8 @@ constexpr int fused_min_blocks()
 // ({L0, L1, L2, NV} of `tmap`, the input state's hydro planes) issued by one
 // thread into the face buffer, which phase 2 overwrites only after phase 1
 // has read it; otherwise every thread loads its cells directly.
-template <int ND, bool EXACT, int TX, int TY, int TZ, int EOSK>
+// NT: threads of the CTA; more than the tile's cells in the wide variant.
+template <int ND, bool EXACT, int TX, int TY, int TZ, int EOSK, int NT>
 __device__ __forceinline__ void fused_step_body(const GridDev& g, const StateDev& in, const StateDev& out, StepCtl* ctl,
                                                 const RunParamsDev& rp, int slot, int out_buf,
                                                 const CUtensorMap* tmap = nullptr, int tma = 0)
@@ -354,7 +355,7 @@ __device__ __forceinline__ void fused_step_body(const GridDev& g, const StateDev
     using S = Shape<ND, TX, TY, TZ>;
     using R = std::conditional_t<EXACT, double, float>;
     constexpr int NV = S::NV;
-    constexpr int NT = S::TVOL;
+    static_assert(NT >= S::TVOL && NT % 32 == 0, "one thread per cell");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     R* sp = reinterpret_cast<R*>(smem_raw);     // [NV][NP] primitives
     R* sa = sp + NV * S::NP;                    // faces: per d [2][NV][A_d]
@@ -365,6 +366,51 @@ __device__ __forceinline__ void fused_step_body(const GridDev& g, const StateDev
     auto sxa = [&](int d) { return sx + nfx * (S::NP + 2 * (S::Aoff(d) / (2 * NV))); };
 
     const int tid = threadIdx.x;
+    // tile origin and the staged box: on its way before the time-loop control
+    // is read
+    int ntile[3], tc[3];
+    ntile[0] = (g.nx[0] + S::T0 - 1) / S::T0;
+    ntile[1] = (g.nx[1] + S::T1 - 1) / S::T1;
+    {
+        int b = blockIdx.x;
+        tc[0] = b % ntile[0];
+        b /= ntile[0];
+        tc[1] = b % ntile[1];
+        tc[2] = b / ntile[1];
+    }
+    const int t0[3] = {tc[0] * S::T0, tc[1] * S::T1, tc[2] * S::T2};
+    const int gorg[3] = {g.ng + t0[0], ND >= 2 ? g.ng + t0[1] : 0, ND >= 3 ? g.ng + t0[2] : 0};
+    int nvalid[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const int tdim = S::T(d);
+        nvalid[d] = d < ND ? min(tdim, g.nx[d] - t0[d]) : 1;
+    }
+
+    // The box lands at the first 128-byte boundary of the face buffer (the
+    // alignment a tensor copy's shared-memory destination needs; the dynamic
+    // shared memory itself starts after the kernel's static shared memory).
+    static_assert(NV * S::NP * sizeof(double) + 128 <= (S::A_TOTAL + S::F_TOTAL) * sizeof(R),
+                  "the staged box fits the face and flux buffers");
+    const unsigned sa_s = smem_u32(sa);
+    double* stage = reinterpret_cast<double*>(reinterpret_cast<unsigned char*>(sa) + ((128u - (sa_s & 127u)) & 127u));
+    // uniform over the CTA: the destination and the box's x origin are aligned
+    // as a tensor copy needs them, else the direct loads run
+    const bool staged = ND >= 2 && tma && (smem_u32(stage) & 127u) == 0u && ((gorg[0] - 2) & 1) == 0;
+    __shared__ uint64_t tile_bar;
+    if constexpr (ND >= 2) {
+        if (staged && tid == 0) {
+            mbar_init(&tile_bar, 1);
+            mbar_init_fence();
+            mbar_arrive_expect_tx(&tile_bar, (unsigned)(NV * S::NP * sizeof(double)));
+            if constexpr (ND == 2) {
+                tma_load_3d(stage, tmap, &tile_bar, gorg[0] - 2, gorg[1] - 2, 0);
+            } else {
+                tma_load_4d(stage, tmap, &tile_bar, gorg[0] - 2, gorg[1] - 2, gorg[2] - 2, 0);
+            }
+        }
+    }
+
     const Decision dec = decide(ctl, slot, rp);
     if (blockIdx.x == 0 && tid == 0) {
         // publish the state seen by step slot+1 (slots other than the ones read)
@@ -399,72 +445,26 @@ __device__ __forceinline__ void fused_step_body(const GridDev& g, const StateDev
         }
         ctl->inv_dt_bits[(slot + 2) % 3] = 0ull;
     }
+    bool arrived = true;
+    if (staged) {
+        __syncthreads(); // the barrier is initialised
+        arrived = mbar_wait_bounded(&tile_bar, 0);
+    }
     if (dec.noop || dec.neg_dt) {
         return;
     }
     const double dt = dec.dt;
     const double dth = dt / 2; // main.cpp:431
 
-    // tile origin (tile-local interior cell (0,0,0) at global (gi0, gj0, gk0))
-    int ntile[3], tc[3];
-    ntile[0] = (g.nx[0] + S::T0 - 1) / S::T0;
-    ntile[1] = (g.nx[1] + S::T1 - 1) / S::T1;
-    {
-        int b = blockIdx.x;
-        tc[0] = b % ntile[0];
-        b /= ntile[0];
-        tc[1] = b % ntile[1];
-        tc[2] = b / ntile[1];
-    }
-    const int t0[3] = {tc[0] * S::T0, tc[1] * S::T1, tc[2] * S::T2};
-    const int gorg[3] = {g.ng + t0[0], ND >= 2 ? g.ng + t0[1] : 0, ND >= 3 ? g.ng + t0[2] : 0};
-    int nvalid[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        const int tdim = S::T(d);
-        nvalid[d] = d < ND ? min(tdim, g.nx[d] - t0[d]) : 1;
-    }
-
     const exact::Eos eeos = exact::make_eos(g.gamma, g.gamma_m1, g.mmw, EOSK);
     const fast::Eos feos{(float)g.gamma, (float)g.gamma_m1, (float)(1.0 / g.gamma_m1)};
 
     // ---- phase 1: state tile + halo -> primitives --------------------------
-    // The box lands at the first 128-byte boundary of the face buffer (the
-    // alignment a tensor copy's shared-memory destination needs; the dynamic
-    // shared memory itself starts after the kernel's static shared memory).
-    static_assert(NV * S::NP * sizeof(double) + 128 <= (S::A_TOTAL + S::F_TOTAL) * sizeof(R),
-                  "the staged box fits the face and flux buffers");
-    const unsigned sa_s = smem_u32(sa);
-    double* stage = reinterpret_cast<double*>(reinterpret_cast<unsigned char*>(sa) + ((128u - (sa_s & 127u)) & 127u));
-    bool staged = false;
-    if constexpr (ND >= 2) {
-        // uniform over the CTA: the destination and the box's x origin are
-        // aligned as a tensor copy needs them, else the direct loads run
-        const bool aligned = (smem_u32(stage) & 127u) == 0u && ((gorg[0] - 2) & 1) == 0;
-        if (tma && aligned) {
-            __shared__ uint64_t tile_bar;
-            if (tid == 0) {
-                mbar_init(&tile_bar, 1);
-                mbar_init_fence();
-            }
-            __syncthreads();
-            if (tid == 0) {
-                mbar_arrive_expect_tx(&tile_bar, (unsigned)(NV * S::NP * sizeof(double)));
-                if constexpr (ND == 2) {
-                    tma_load_3d(stage, tmap, &tile_bar, gorg[0] - 2, gorg[1] - 2, 0);
-                } else {
-                    tma_load_4d(stage, tmap, &tile_bar, gorg[0] - 2, gorg[1] - 2, gorg[2] - 2, 0);
-                }
-            }
-            staged = true;
-            const bool arrived = mbar_wait_bounded(&tile_bar, 0);
-            if (__syncthreads_or(!arrived) && tid == 0) {
-                // the box never arrived: stop the run with HCL_ERR_TIMEOUT
-                ctl->err = 6;
-                ctl->errflag[(slot + 1) & 1] = 1;
-                ctl->final_buf = out_buf;
-            }
-        }
+    if (staged && __syncthreads_or(!arrived) && tid == 0) {
+        // the box never arrived: stop the run with HCL_ERR_TIMEOUT
+        ctl->err = 6;
+        ctl->errflag[(slot + 1) & 1] = 1;
+        ctl->final_buf = out_buf;
     }
     for (int p = tid; p < S::NP; p += NT) {
         const int lx = p % S::L0;
@@ -514,6 +514,18 @@ __device__ __forceinline__ void fused_step_body(const GridDev& g, const StateDev
         }
         for (int f = 0; f < nfx; ++f) {
             sx[f * S::NP + p] = (R)__ldg(in.q + o + in.plane * (NV + f));
+        }
+    }
+    // the wide variant has the registers to load its cell's old state now
+    double q_pre[NV];
+    if constexpr (NT > S::TVOL) {
+        const int x0 = tid % S::T0, x1 = (tid / S::T0) % S::T1, x2 = tid / (S::T0 * S::T1);
+        if (tid < S::TVOL && x0 < nvalid[0] && x1 < nvalid[1] && x2 < nvalid[2]) {
+            const int64_t so = sidx(in, g.n[1], gorg[0] + x0, ND >= 2 ? gorg[1] + x1 : 0, ND >= 3 ? gorg[2] + x2 : 0);
+#pragma unroll
+            for (int v = 0; v < NV; ++v) {
+                q_pre[v] = in.q[so + in.plane * v];
+            }
         }
     }
     __syncthreads();
@@ -881,11 +893,15 @@ __device__ __forceinline__ void fused_step_body(const GridDev& g, const StateDev
     __syncthreads();
 
     // ---- phase 3: one Riemann solve per face --------------------------------
-#pragma unroll
-    for (int d = 0; d < ND; ++d) {
-        const R* base = sa + S::Aoff(d);
-        R* fbase = sf + S::Foff(d);
-        for (int f = tid; f < S::Fsize(d); f += NT) {
+    // (the dimensions' faces in one list, each padded to whole warps)
+    auto solve_face = [&](auto dc, int f) {
+        constexpr int d = decltype(dc)::value;
+        if constexpr (d < ND) {
+            if (f >= S::Fsize(d)) {
+                return;
+            }
+            const R* base = sa + S::Aoff(d);
+            R* fbase = sf + S::Foff(d);
             const int fx0 = f % S::Fdim(d, 0);
             const int fx1 = (f / S::Fdim(d, 0)) % S::Fdim(d, 1);
             const int fx2 = f / (S::Fdim(d, 0) * S::Fdim(d, 1));
@@ -908,6 +924,18 @@ __device__ __forceinline__ void fused_step_body(const GridDev& g, const StateDev
             for (int v = 0; v < NV; ++v) {
                 fbase[v * S::Fsize(d) + f] = fl[v];
             }
+        }
+    };
+    constexpr int P0 = (S::Fsize(0) + 31) / 32 * 32;
+    constexpr int P1 = ND >= 2 ? (S::Fsize(1) + 31) / 32 * 32 : 0;
+    constexpr int P2 = ND >= 3 ? (S::Fsize(2) + 31) / 32 * 32 : 0;
+    for (int f = tid; f < P0 + P1 + P2; f += NT) {
+        if (f < P0) {
+            solve_face(std::integral_constant<int, 0>{}, f);
+        } else if (f < P0 + P1) {
+            solve_face(std::integral_constant<int, 1>{}, f - P0);
+        } else {
+            solve_face(std::integral_constant<int, 2>{}, f - P0 - P1);
         }
     }
     __syncthreads();
@@ -1010,7 +1038,7 @@ __device__ __forceinline__ void fused_step_body(const GridDev& g, const StateDev
         double q[NV];
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
-            q[v] = in.q[so + in.plane * v];
+            q[v] = NT > S::TVOL ? q_pre[v] : in.q[so + in.plane * v];
         }
         const int64_t cgl = lidx(g, gi, gj, gk);
         double qn[NV];
@@ -1223,25 +1251,27 @@ __device__ __forceinline__ void fused_step_body(const GridDev& g, const StateDev
             ctl->final_buf = out_buf;
         }
 
-        // store + ghost images
-        int pos[3][9];
-        int flp[3][9];
-        int cnt[3] = {1, 1, 1};
+        // store + ghost images: bit 0 of a mask is the cell itself, bit 1 + k the
+        // ghost slot k it fills
         const int gidx[3] = {gi, gj, gk};
+        unsigned img[3] = {0u, 0u, 0u};
 #pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            pos[d][0] = gidx[d];
-            flp[d][0] = 0;
-            if (d < ND) {
-                cnt[d] += ghost_images(gidx[d], g.n[d], g.ng, g.bc[2 * d], g.bc[2 * d + 1], &pos[d][1], &flp[d][1]);
-            }
+        for (int d = 0; d < ND; ++d) {
+            img[d] = ghost_mask(gidx[d], g.n[d], g.ng, g.bc[2 * d], g.bc[2 * d + 1]);
         }
-        for (int a2 = 0; a2 < cnt[2]; ++a2) {
-            for (int a1 = 0; a1 < cnt[1]; ++a1) {
-                for (int a0 = 0; a0 < cnt[0]; ++a0) {
-                    const int pi = pos[0][a0], pj = pos[1][a1], pk = pos[2][a2];
+        auto image = [&](int d, unsigned bit, int* flip) {
+            const int k = __ffs(bit) - 1;
+            *flip = k && ((img[d] >> (15 + k)) & 1u);
+            return k ? ghost_slot(k - 1, g.n[d], g.ng) : gidx[d];
+        };
+        int fl[3];
+        for (unsigned b2 = (img[2] & 0xffffu) << 1 | 1u; b2; b2 &= b2 - 1u) {
+            const int pk = image(2, b2, &fl[2]);
+            for (unsigned b1 = (img[1] & 0xffffu) << 1 | 1u; b1; b1 &= b1 - 1u) {
+                const int pj = image(1, b1, &fl[1]);
+                for (unsigned b0 = (img[0] & 0xffffu) << 1 | 1u; b0; b0 &= b0 - 1u) {
+                    const int pi = image(0, b0, &fl[0]);
                     const int64_t oo = sidx(out, g.n[1], pi, pj, pk);
-                    const int fl[3] = {flp[0][a0], flp[1][a1], flp[2][a2]};
                     out.q[oo] = qn[0];
 #pragma unroll
                     for (int d = 0; d < ND; ++d) {
@@ -1268,7 +1298,9 @@ __device__ __forceinline__ void fused_step_body(const GridDev& g, const StateDev
                     } else {
 #pragma unroll
                         for (int d = 0; d < ND; ++d) {
-                            cell += (inv_rho_u[d] + sound) / dxg[d];
+                            const double a = inv_rho_u[d] + sound;
+                            const q64::Den w = q64::den(dxg[d]);
+                            cell += EXACT && q64::within(a) && q64::den_ok(w.b) ? q64::quo(a, w) : a / w.b;
                         }
                     }
                     if (isnan(cell)) {
@@ -1338,10 +1370,12 @@ __device__ __forceinline__ void fused_step_body(const GridDev& g, const StateDev
                 }
                 double v = xn / qn[0];
                 v = v < 0. ? 0. : (v > 1. ? 1. : v);
-                for (int a2 = 0; a2 < cnt[2]; ++a2) {
-                    for (int a1 = 0; a1 < cnt[1]; ++a1) {
-                        for (int a0 = 0; a0 < cnt[0]; ++a0) {
-                            out.q[sidx(out, g.n[1], pos[0][a0], pos[1][a1], pos[2][a2]) + out.plane * (NV + f)] = v;
+                for (unsigned b2 = (img[2] & 0xffffu) << 1 | 1u; b2; b2 &= b2 - 1u) {
+                    const int pk = image(2, b2, &fl[2]);
+                    for (unsigned b1 = (img[1] & 0xffffu) << 1 | 1u; b1; b1 &= b1 - 1u) {
+                        const int pj = image(1, b1, &fl[1]);
+                        for (unsigned b0 = (img[0] & 0xffffu) << 1 | 1u; b0; b0 &= b0 - 1u) {
+                            out.q[sidx(out, g.n[1], image(0, b0, &fl[0]), pj, pk) + out.plane * (NV + f)] = v;
                         }
                     }
                 }
@@ -1359,7 +1393,7 @@ __device__ __forceinline__ void fused_step_body(const GridDev& g, const StateDev
     }
     __syncthreads();
     if (w == 0) {
-        m = lane < (NT + 31) / 32 ? red[lane] : 0.0;
+        m = lane < NT / 32 ? red[lane] : 0.0;
         m = warp_max_d(m);
         if (lane == 0) {
             atomicMax(&ctl->inv_dt_bits[(slot + 1) % 3], dbl_bits(m));
@@ -1375,7 +1409,22 @@ __global__ void __launch_bounds__(TX*(ND >= 2 ? TY : 1)*(ND >= 3 ? TZ : 1))
 k_fused_step(GridDev g, StateDev in, StateDev out, StepCtl* ctl, RunParamsDev rp, int slot, int out_buf,
              const __grid_constant__ CUtensorMap tmap, int tma)
 {
-    fused_step_body<ND, EXACT, TX, TY, TZ, EOSK>(g, in, out, ctl, rp, slot, out_buf, &tmap, tma);
+    fused_step_body<ND, EXACT, TX, TY, TZ, EOSK, Shape<ND, TX, TY, TZ>::TVOL>(g, in, out, ctl, rp, slot, out_buf, &tmap,
+                                                                             tma);
+}
+
+// The 16 x 16 tile with a thread for every item of a phase, for grids of at
+// most one tile per SM, whose step is the latency of one tile: 320 cells with
+// faces and 544 faces fit one round (FP32-mixed, 576 threads) or one and two
+// (FP64, 352 threads, 184 registers) instead of two and three.
+template <bool EXACT>
+constexpr int kWideThreads = EXACT ? 352 : 576;
+template <bool EXACT, int EOSK = EOS_PERFECT_GAS>
+__global__ void __launch_bounds__(kWideThreads<EXACT>, 1)
+k_fused_step_wide(GridDev g, StateDev in, StateDev out, StepCtl* ctl, RunParamsDev rp, int slot, int out_buf,
+                  const __grid_constant__ CUtensorMap tmap, int tma)
+{
+    fused_step_body<2, EXACT, 16, 16, 1, EOSK, kWideThreads<EXACT>>(g, in, out, ctl, rp, slot, out_buf, &tmap, tma);
 }
 
 // the same step with the occupancy bound above (instantiated where it is > 0)
@@ -1385,7 +1434,8 @@ __global__ void __launch_bounds__(TX*(ND >= 2 ? TY : 1)*(ND >= 3 ? TZ : 1),
 k_fused_step_occ(GridDev g, StateDev in, StateDev out, StepCtl* ctl, RunParamsDev rp, int slot, int out_buf,
                  const __grid_constant__ CUtensorMap tmap, int tma)
 {
-    fused_step_body<ND, EXACT, TX, TY, TZ, EOSK>(g, in, out, ctl, rp, slot, out_buf, &tmap, tma);
+    fused_step_body<ND, EXACT, TX, TY, TZ, EOSK, Shape<ND, TX, TY, TZ>::TVOL>(g, in, out, ctl, rp, slot, out_buf, &tmap,
+                                                                             tma);
 }
 
 template <int ND, bool EXACT, int TX, int TY, int TZ>
@@ -1404,8 +1454,17 @@ struct FusedLauncher {
     // occupancy); called once per process before any launch (never during
     // stream capture).
     static constexpr int kMinBlocks = fused_min_blocks<ND, EXACT, TX, TY, TZ>();
+    static constexpr bool kWide = ND == 2 && TX == 16 && TY == 16;
+    template <int EOSK>
+    static void configure_wide()
+    {
+        if constexpr (kWide) {
+            set_max_dynamic(reinterpret_cast<const void*>(k_fused_step_wide<EXACT, EOSK>));
+        }
+    }
     static void configure()
     {
+        configure_wide<EOS_PERFECT_GAS>();
         set_max_dynamic(reinterpret_cast<const void*>(k_fused_step<ND, EXACT, TX, TY, TZ>));
         if constexpr (EXACT) {
             set_max_dynamic(reinterpret_cast<const void*>(k_fused_step<ND, EXACT, TX, TY, TZ, EOS_RAD_GAS>));
@@ -1416,6 +1475,17 @@ struct FusedLauncher {
                 set_max_dynamic(reinterpret_cast<const void*>(k_fused_step_occ<ND, EXACT, TX, TY, TZ, EOS_RAD_GAS>));
             }
         }
+    }
+    static int sm_count()
+    {
+        static PerDevice cache;
+        int dev = 0;
+        cudaGetDevice(&dev);
+        return cache.get(dev, [dev] {
+            int v = 0;
+            cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+            return v;
+        });
     }
     // the occupancy-bounded kernel pays off when that many CTAs fit the SM's
     // shared memory (1 KB reserved per CTA, up to 512 B static)
@@ -1462,6 +1532,14 @@ struct FusedLauncher {
         std::memset(&map, 0, sizeof(map));
         const int box[3] = {S::L0, S::L1, S::L2};
         const int tma = (ND >= 2 && g.ng % 2 == 0 && encode_tile_map(g, in, S::NV, box, &map)) ? 1 : 0;
+        if constexpr (kWide && EOSK != EOS_RAD_GAS) {
+            if (blocks <= sm_count()) {
+                k_fused_step_wide<EXACT, EOSK>
+                    <<<blocks, kWideThreads<EXACT>, sm, s>>>(g, in, out, ctl, rp, slot, out_buf, map, tma);
+                ++g_launches;
+                return;
+            }
+        }
         if (use_occ(g.nfx)) {
             k_fused_step_occ<ND, EXACT, TX, TY, TZ, EOSK>
                 <<<blocks, S::TVOL, sm, s>>>(g, in, out, ctl, rp, slot, out_buf, map, tma);
@@ -1486,6 +1564,7 @@ struct FusedLauncher {
     static void configure_fast()
     {
         static_assert(EXACT, "fast FP64 runs the FP64 kernels");
+        configure_wide<EOS_PERFECT_GAS_FAST>();
         set_max_dynamic(reinterpret_cast<const void*>(k_fused_step<ND, EXACT, TX, TY, TZ, EOS_PERFECT_GAS_FAST>));
         if constexpr (kMinBlocks > 0) {
             set_max_dynamic(reinterpret_cast<const void*>(k_fused_step_occ<ND, EXACT, TX, TY, TZ, EOS_PERFECT_GAS_FAST>));

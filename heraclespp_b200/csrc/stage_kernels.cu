@@ -892,7 +892,7 @@ void dispatch_nd(int nd, F&& f)
 // while its other warps bring in the products rho dv of the next chunks through
 // registers and shared memory, two chunks ahead of the sum.  One thread per
 // shell that loads for itself waits out each load: 954 us; loads not issued
-// ahead: 169 us; so: 84 us.  The shells' volumes do not change and come from the host
+// ahead: 169 us; so: 57 us.  The shells' volumes do not change and come from the host
 // (g.shell_dv).
 constexpr int kShellWarps = 16;
 constexpr int kShellChunk = 96; // 2 buffers x 96 x 32 doubles = 48 KB
