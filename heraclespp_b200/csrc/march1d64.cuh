@@ -409,6 +409,22 @@ __global__ void __launch_bounds__(kM1MaxThreads, 1) k_march1d64(GridDev g, State
     cl.sync(); // no CTA leaves while another may still write to its shared memory
 }
 
+inline cudaLaunchConfig_t march1d64_config(int ctas, int threads, cudaStream_t s, cudaLaunchAttribute* at)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = sizeof(M1Shared);
+    cfg.stream = s;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = ctas;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
 template <int KIND>
 bool march1d64_configure_t()
 {
@@ -416,10 +432,16 @@ bool march1d64_configure_t()
     int dev = 0;
     cudaGetDevice(&dev);
     return cache.get(dev, [] {
+        // the largest cluster must fit this device (or the part of it in use)
+        cudaLaunchAttribute at[1];
+        cudaLaunchConfig_t cfg = march1d64_config(kM1MaxCtas, kM1MaxThreads, nullptr, at);
+        int clusters = 0;
         const bool ok = cudaFuncSetAttribute(k_march1d64<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)sizeof(M1Shared)) == cudaSuccess &&
                         cudaFuncSetAttribute(k_march1d64<KIND>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
-                            cudaSuccess;
+                            cudaSuccess &&
+                        cudaOccupancyMaxActiveClusters(&clusters, k_march1d64<KIND>, &cfg) == cudaSuccess && clusters > 0;
+        cudaGetLastError();
         return ok ? 1 : 0;
     }) != 0;
 }
@@ -437,18 +459,9 @@ void march1d64_launch_t(const GridDev& g, const StateDev& st0, const StateDev& s
 {
     const int chunk = march1d64_chunk(g);
     const int ctas = (g.nx[0] + chunk - 1) / chunk;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(ctas);
-    cfg.blockDim = dim3(std::min(chunk, kM1MaxThreads - 32) + 32); // the halo's cells in the same round
-    cfg.dynamicSmemBytes = sizeof(M1Shared);
-    cfg.stream = s;
+    // one thread per cell and the halo's in the same round
     cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = ctas;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cudaLaunchConfig_t cfg = march1d64_config(ctas, std::min(chunk, kM1MaxThreads - 32) + 32, s, at);
     cudaLaunchKernelEx(&cfg, k_march1d64<KIND>, g, st0, st1, ctl, rp, slot0, steps, chunk);
     ++g_launches;
 }

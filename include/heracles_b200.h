@@ -269,6 +269,8 @@ typedef struct hcl_run_result {
 /* Runs the reference time loop (main.cpp:354-531) with the fused step kernel,
  * everything on the device: CFL dt reduced inside the step kernel, dt clamps,
  * health check and ghost filling in place; steps are replayed from CUDA graphs.
+ * FP64 1-D domains of up to 8192 cells (perfect gas, no scalars, pressure fix or
+ * internal-mass gravity) instead take up to 4096 steps per launch.
  * Synchronises at the end (and between graph chunks when nsteps <= 0).
  * Passive scalars (nfx > 0) and the pressure fix ride in the fused
  * shared-memory tile kernels (FP64, fast FP64 and FP32-mixed, which applies
