@@ -20,6 +20,13 @@
 // 168 registers).  8 warps: 5 % slower; 16 (128 registers): as fast in the
 // exact form, 11 % slower in the fast one.  Fast FP64, 1333 x 1001, Minmod:
 // 0.19 -> 0.12 ms.
+//
+// Gas at rest: zero differences and momenta stay on the straight-line path
+// (512^2 blast, Minmod and HLL, 47 us per step as with noise in every cell; 93 us
+// when each zero asked for a second look).  A front's tail, momenta from 2^-800
+// down to the smallest numbers, is done again out of line; a strip that it crosses
+// in every row takes 2.4 times a plain one, and the step waits for it: Gresho
+// 512^2 88 us (141 us with plain divisions one by one, tile kernel 99 us).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -38,20 +45,59 @@ constexpr int kMarchLanesOut = 28;
 constexpr int kMarchWarps = 12;
 constexpr int kMarchRingDoubles = 8 * 4 * 32; // 8 row slots x 4 variables x 32 lanes per warp
 
-template <int KIND>
-static __device__ __noinline__ void quotients_slow(const double* a, double bx, double by, double* q)
+// The slopes of a row with tiny or extreme data, by the whole warp (a lane's
+// left quotient is its neighbour's): the differences a (x, then y), their
+// widths (h_ok: in range), the lower y quotients low.  Gives the quotients q and
+// the products s of the slopes and half the widths.
+template <int LIM>
+static __device__ __noinline__ void slopes_slow(const double* a, q64::Den hx, q64::Den hy, bool h_ok, const double* low,
+                                                double dlx, double dly, double* q, double* s)
 {
-    for (int v = 0; v < 4; ++v) {
-        q[v] = a[v] / bx;
-        q[4 + v] = a[4 + v] / by;
+    double Q[8], S[8];
+    bool good = h_ok;
+#pragma unroll
+    for (int v = 0; v < 8; ++v) {
+        Q[v] = q64::quo_tiny(a[v], v < 4 ? hx : hy, good);
+    }
+#pragma unroll
+    for (int v = 0; v < 8; ++v) {
+        q[v] = Q[v];
+    }
+    if (!good) {
+        for (int v = 0; v < 8; ++v) {
+            q[v] = a[v] / (v < 4 ? hx.b : hy.b);
+        }
+    }
+    unsigned bad = 0u;
+#pragma unroll
+    for (int v = 0; v < 8; ++v) {
+        const double R = q[v];
+        const double L = v < 4 ? __shfl_up_sync(0xffffffffu, R, 1) : low[v - 4];
+        bool pair;
+        S[v] = exact::limited_width<LIM>(v < 4 ? dlx : dly) * exact::limited_tiny<LIM>(R, L, pair);
+        bad |= (unsigned)!pair << v;
+    }
+#pragma unroll
+    for (int v = 0; v < 8; ++v) {
+        s[v] = S[v];
+    }
+    if (__any_sync(0xffffffffu, bad != 0u)) {
+        for (int v = 0; v < 8; ++v) {
+            const double L = v < 4 ? __shfl_up_sync(0xffffffffu, q[v], 1) : low[v & 3];
+            if (bad >> v & 1u) {
+                s[v] = ((v < 4 ? dlx : dly) / 2) * exact::plain::slope(LIM, q[v], L);
+            }
+        }
     }
 }
-// the products (dl/2) * slope of 8 quotient pairs
-template <int LIM, int KIND>
-static __device__ __noinline__ void slopes_slow(const double* R, const double* L, double wx, double wy, double* s)
+// the same products in the fast forms, from the quotients
+template <int LIM>
+static __device__ __noinline__ void slopes_slow_fast(const double* R, const double* L, double wx, double wy, double* s)
 {
     for (int v = 0; v < 8; ++v) {
-        s[v] = (v < 4 ? wx : wy) * exact::plain::slope(LIM, R[v], L[v], KIND);
+        if (!exact::limited_fast_ok<LIM>(R[v], L[v])) {
+            s[v] = (v < 4 ? wx : wy) * exact::plain::slope(LIM, R[v], L[v], EOS_PERFECT_GAS_FAST);
+        }
     }
 }
 
@@ -64,7 +110,7 @@ __device__ __forceinline__ q64::Den face_width(bool unif, double dl, double dl_p
         return q64::Den{1.0, 1.0};
     }
     const double h = (dl + dl_p) / 2;
-    return FAST ? q64::Den{h, 1.0 / h} : q64::den(h);
+    return FAST ? q64::Den{h, 1.0 / h} : q64::den_any(h);
 }
 
 template <int LIM, int RS, int KIND>
@@ -105,7 +151,7 @@ __device__ __forceinline__ void march2d_strip(const GridDev& g, const double* __
     const bool unif = FAST && g.uniform_cart;
     const q64::Den hx = face_width<FAST>(unif, g.dx[0][gq], g.dx[0][gq + 1]);
     const double wx = unif ? (LIM == LIM_VANLEER ? 1.0 : 0.5) : exact::limited_width<LIM>(dlx);
-    const bool hx_ok = FAST || q64::den_ok(hx.b);
+    const bool hx_ok = FAST || q64::width_ok(hx.b);
     const q64::Den dcol = q64::den(g.dx[0][colc]);
     const double ds1 = dlx * dx2;
     const double gvx = gravity_at(g, gx, 0);
@@ -166,7 +212,7 @@ __device__ __forceinline__ void march2d_strip(const GridDev& g, const double* __
         // this cell; the left ones come from the next lane and the last row
         double R[8], Lq[8], s[8];
         const q64::Den hy = face_width<FAST>(unif, dly, g.dx[1][jn]);
-        const bool h_ok = hx_ok && (FAST || q64::den_ok(hy.b));
+        const bool h_ok = hx_ok && (FAST || q64::width_ok(hy.b));
         const double wy = unif ? wx : exact::limited_width<LIM>(dly);
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
@@ -175,7 +221,7 @@ __device__ __forceinline__ void march2d_strip(const GridDev& g, const double* __
             R[v] = FAST ? ax * hx.y : q64::quo(ax, hx);
             R[4 + v] = FAST ? ay * hy.y : q64::quo(ay, hy);
         }
-        q64::Range Z(h_ok);
+        q64::Range S(h_ok);
 #pragma unroll
         for (int v = 0; v < 8; ++v) {
             Lq[v] = v < 4 ? __shfl_up_sync(FULL, R[v], 1) : yq[v - 4];
@@ -183,59 +229,56 @@ __device__ __forceinline__ void march2d_strip(const GridDev& g, const double* __
             if constexpr (LIM == LIM_CONSTANT) {
                 s[v] = 0.0;
             } else if constexpr (FAST) {
-                s[v] = w * exact::limited_fast<LIM>(R[v], Lq[v], Z);
+                s[v] = w * exact::limited_fast<LIM>(R[v], Lq[v], S);
             } else {
-                s[v] = w * exact::limited_core<LIM>(R[v], Lq[v], Z);
+                s[v] = w * exact::limited_core<LIM>(R[v], Lq[v], S);
             }
         }
         if constexpr (LIM != LIM_CONSTANT) {
-            bool ok = true;
+            const bool again = in_use && !S.ok();
             if constexpr (FAST) {
-                if (!Z.ok()) {
+                if (again) {
+                    double Rt[8], Lt[8], st[8];
 #pragma unroll
                     for (int v = 0; v < 8; ++v) {
-                        ok = ok && exact::limited_fast_ok<LIM>(R[v], Lq[v]);
+                        Rt[v] = R[v];
+                        Lt[v] = Lq[v];
+                        st[v] = s[v];
+                    }
+                    slopes_slow_fast<LIM>(Rt, Lt, unif ? 0.5 : dlx / 2, unif ? 0.5 : dly / 2, st);
+#pragma unroll
+                    for (int v = 0; v < 8; ++v) {
+                        s[v] = st[v];
                     }
                 }
-            } else if (__any_sync(FULL, in_use && !Z.ok())) {
-                // flat or extreme data somewhere in the row: the quotients
-                // first (a neighbour's too, hence warp-wide), then the slopes
-                double at[8];
-                bool q_ok = h_ok;
+            } else if (__any_sync(FULL, again)) {
+                double at[8], lt[4], qt[8], st[8];
+                bool low_ok = true;
 #pragma unroll
                 for (int v = 0; v < 4; ++v) {
                     at[v] = __shfl_down_sync(FULL, wc[v], 1) - wc[v];
                     at[4 + v] = wn[v] - wc[v];
-                    q_ok = q_ok && q64::within0(at[v]) && q64::within0(at[4 + v]);
+                    lt[v] = yq[v];
+                    low_ok = low_ok && q64::num_ok(yq[v]);
                 }
-                if (!q_ok) {
-                    double qt[8];
-                    quotients_slow<KIND>(at, hx.b, hy.b, qt);
+                if (!low_ok) {
+                    // a tiny lower y quotient may be off: row j-1 is still staged
+                    double qm[4], wm[4];
 #pragma unroll
-                    for (int v = 0; v < 8; ++v) {
-                        R[v] = qt[v];
+                    for (int v = 0; v < 4; ++v) {
+                        qm[v] = ring[(j - 1) & 7][v][lane];
+                    }
+                    exact::to_prim_slow<2, KIND>(e, qm, wm);
+                    const double hm = (g.dx[1][j - 1] + dly) / 2;
+#pragma unroll
+                    for (int v = 0; v < 4; ++v) {
+                        lt[v] = (wc[v] - wm[v]) / hm;
                     }
                 }
-                ok = __shfl_up_sync(FULL, (int)q_ok, 1) && q_ok;
+                slopes_slow<LIM>(at, hx, hy, h_ok, lt, dlx, dly, qt, st);
 #pragma unroll
                 for (int v = 0; v < 8; ++v) {
-                    if (v < 4) {
-                        Lq[v] = __shfl_up_sync(FULL, R[v], 1);
-                    }
-                    ok = ok && exact::limited_ok<LIM>(R[v], Lq[v]);
-                }
-            }
-            if (!ok) {
-                double Rt[8], Lt[8], st[8];
-#pragma unroll
-                for (int v = 0; v < 8; ++v) {
-                    Rt[v] = R[v];
-                    Lt[v] = Lq[v];
-                }
-                // (dl / 2) times the plain slope (raw differences: 1/2)
-                slopes_slow<LIM, KIND>(Rt, Lt, unif ? 0.5 : dlx / 2, unif ? 0.5 : dly / 2, st);
-#pragma unroll
-                for (int v = 0; v < 8; ++v) {
+                    R[v] = qt[v];
                     s[v] = st[v];
                 }
             }

@@ -115,7 +115,7 @@ k_march3d64(GridDev g, StateDev in, StateDev out, StepCtl* ctl, RunParamsDev rp,
         const bool x = k < kM3PX;
         const int d = x ? 0 : 1;
         const int c = min((x ? i0 - 2 + k : j0 - 2 + k - kM3PX), g.n[d] - 2);
-        const q64::Den h = raw ? q64::Den{1.0, 1.0} : q64::den((g.dx[d][c] + g.dx[d][c + 1]) / 2);
+        const q64::Den h = raw ? q64::Den{1.0, 1.0} : q64::den_any((g.dx[d][c] + g.dx[d][c + 1]) / 2);
         (x ? sh.hx[k] : sh.hy[k - kM3PX]) = h;
     }
 
@@ -204,8 +204,8 @@ k_march3d64(GridDev g, StateDev in, StateDev out, StepCtl* ctl, RunParamsDev rp,
                     hL = sh.hy[w];
                     hR = sh.hy[w + 1];
                 } else {
-                    hL = raw ? q64::Den{1.0, 1.0} : q64::den((g.dx[2][z - 1] + dlz) / 2);
-                    hR = raw ? q64::Den{1.0, 1.0} : q64::den((dlz + g.dx[2][z + 1]) / 2);
+                    hL = raw ? q64::Den{1.0, 1.0} : q64::den_any((g.dx[2][z - 1] + dlz) / 2);
+                    hR = raw ? q64::Den{1.0, 1.0} : q64::den_any((dlz + g.dx[2][z + 1]) / 2);
                 }
                 if constexpr (LIM == LIM_CONSTANT) {
 #pragma unroll
@@ -369,7 +369,7 @@ k_march3d64(GridDev g, StateDev in, StateDev out, StepCtl* ctl, RunParamsDev rp,
                 double uL[5], uR[5], F[5];
 #pragma unroll
                 for (int v = 0; v < 5; ++v) {
-                    uL[v] = sh.face[1][v][max(tid - 1, 0)];
+                    uL[v] = sh.face[1][v][lane ? tid - 1 : tid]; // lane 0 has no left face
                     uR[v] = sh.face[0][v][tid];
                 }
                 const int64_t o = z * plane2 + (int64_t)min(row, n1 - 1) * in.pitch + min(col, n0 - 1);

@@ -26,7 +26,8 @@ struct Eos {
     double gamma, gamma_m1, mmw;
     int kind; // EOS_PERFECT_GAS, EOS_RAD_GAS or EOS_PERFECT_GAS_FAST
     // the perfect gas's constant denominators (perfect_gas.hpp:46-83): mu m_p
-    // and mu m_p (gamma - 1); consts_ok: both usable as such
+    // and mu m_p (gamma - 1); consts_ok: both usable as such, and the internal
+    // energy not far below the pressure
     q64::Den mk, ev;
     bool consts_ok;
 };
@@ -35,7 +36,8 @@ __device__ __forceinline__ Eos make_eos(double gamma, double gamma_m1, double mm
 {
     const double b = mmw * kMp;
     const double c = mmw * kMp * gamma_m1;
-    return Eos{gamma, gamma_m1, mmw, kind, q64::Den{b, 1.0 / b}, q64::Den{c, 1.0 / c}, q64::den_ok(b) && q64::den_ok(c)};
+    return Eos{gamma, gamma_m1, mmw, kind, q64::Den{b, 1.0 / b}, q64::Den{c, 1.0 / c},
+               q64::den_ok(b) && q64::den_ok(c) && gamma_m1 <= 1024.0};
 }
 
 __device__ __forceinline__ Eos eos_of(const GridDev& g)
@@ -375,45 +377,48 @@ __device__ __forceinline__ void riemann(const Eos& e, int solver, const double* 
 
 // hydro/euler_equations.hpp:41-59
 using plain::ek_cons;
-using plain::ek_prim;
 
 // ---- the same results with shared reciprocals (quot64.cuh) ------------------
 // Each *_core evaluates a group of expressions straight through and gathers
-// its operands in two ranges: S, and Z for numerators that may be zero.  Where
-// both hold every quotient and root is the rounded one.  Otherwise the caller
-// looks at the Z operands one by one and, unless those outside are all zeros,
-// redoes the group with plain operators, out of line.  Scalings by powers of two (the /2 of the kinetic energy, the 4/2
-// and 2/2 of the limiters) are folded, which is exact in that range.
-template <int ND>
-static __device__ __noinline__ void to_prim_slow(Eos e, const double* c, double* p)
-{
-    plain::to_prim<ND>(e, c, p);
-}
+// its operands in a range S: denominators, pressures, and numerators, which may
+// be zero or smaller.  Where it holds every quotient and root is the rounded
+// one.  Otherwise the group is done again out of line: with quo_tiny() for the
+// numerators (TINY) if those were the matter, else with plain operators.  Scalings by powers of two (the /2 of the kinetic
+// energy, the 4/2 and 2/2 of the limiters) are folded, which is exact in that
+// range.
 template <int ND>
 static __device__ __noinline__ void to_cons_flux_slow(Eos e, const double* p, int l, double* c, double* f)
 {
     plain::to_cons<ND>(e, p, c);
     plain::flux_prim<ND>(e, p, l, f);
 }
-template <int ND>
-static __device__ __noinline__ void riemann_slow(Eos e, int solver, const double* cL, const double* cR, int l, double* f)
-{
-    plain::riemann<ND>(e, solver, cL, cR, l, f);
-}
 static __device__ __noinline__ double sound_slow(Eos e, double rho, double P)
 {
     return plain_sound(e, rho, P);
 }
+// a numerator's quotient
+template <bool TINY>
+__device__ __forceinline__ double num_quo(double a, const q64::Den& d, q64::Range& S)
+{
+    if constexpr (TINY) {
+        bool good = true;
+        const double q = q64::quo_tiny(a, d, good);
+        S.also(good);
+        return q;
+    } else {
+        return q64::quo(a, d);
+    }
+}
 
 // hydro/euler_equations.hpp:111-122.  r, k: the denominators rho and rho kb;
-// evol: the internal energy.  S holds rho and P, Z the momenta.
-template <int ND>
+// evol: the internal energy.  S holds rho, P and the momenta.
+template <int ND, bool TINY = false>
 __device__ __forceinline__ void prim_core(const Eos& e, const double* c, double* p, q64::Den& r, q64::Den& k,
-                                          double& evol, q64::Range& S, q64::Range& Z)
+                                          double& evol, q64::Range& S)
 {
-    r = q64::den(c[0]);
     p[0] = c[0];
     if (e.kind == EOS_PERFECT_GAS_FAST) {
+        r = q64::den(c[0]);
         double mu = 0;
 #pragma unroll
         for (int d = 0; d < ND; ++d) {
@@ -425,38 +430,36 @@ __device__ __forceinline__ void prim_core(const Eos& e, const double* c, double*
         S.add(c[0], p[1 + ND]);
         return;
     }
+    r = q64::den_any(c[0]);
     double norm = 0;
 #pragma unroll
     for (int d = 0; d < ND; ++d) {
         norm += c[1 + d] * c[1 + d];
-        p[1 + d] = q64::quo(c[1 + d], r);
+        p[1 + d] = num_quo<TINY>(c[1 + d], r, S);
     }
     evol = __fma_rn(-0.5, q64::quo(norm, r), c[1 + ND]);
     const double kb = c[0] * kKb;
     k = q64::den_from(kb, r.y * (1 / kKb));
     p[1 + ND] = q64::quo(kb * q64::quo(evol * e.mmw * kMp * e.gamma_m1, k), e.mk);
     S.add(c[0], p[1 + ND]);
-    S.low(c[0]);
     S.low(kb);
-    Z.add(c[1], ND >= 2 ? c[2] : c[1]);
+    S.num(c[1], c[ND >= 2 ? 2 : 1]);
     if constexpr (ND == 3) {
-        Z.add(c[3]);
+        S.num(c[3], c[3]);
     }
 }
-// the Z operands of prim_core
-template <int ND>
-__device__ __forceinline__ bool prim_zeros(const Eos& e, const double* c)
+template <int ND, int KIND>
+static __device__ __noinline__ void to_prim_slow(Eos e, const double* c, double* p)
 {
-    bool ok = true;
-    if (e.kind != EOS_PERFECT_GAS_FAST) {
-#pragma unroll
-        for (int d = 0; d < ND; ++d) {
-            ok = ok && q64::within0(c[1 + d]);
-        }
+    e.kind = KIND;
+    q64::Den r, k;
+    double evol;
+    q64::Range S(e.consts_ok);
+    prim_core<ND, true>(e, c, p, r, k, evol, S);
+    if (!S.dens_ok()) {
+        plain::to_prim<ND>(e, c, p);
     }
-    return ok;
 }
-
 template <int ND>
 __device__ __forceinline__ void to_prim(const Eos& e, const double* c, double* p)
 {
@@ -466,20 +469,22 @@ __device__ __forceinline__ void to_prim(const Eos& e, const double* c, double* p
     }
     q64::Den r, k;
     double evol;
-    q64::Range S(e.consts_ok), Z;
-    prim_core<ND>(e, c, p, r, k, evol, S, Z);
-    if (!(S.ok() && Z.ok())) {
-        if (!(S.ok() && prim_zeros<ND>(e, c))) {
-            double ct[ND + 2], pt[ND + 2];
+    q64::Range S(e.consts_ok);
+    prim_core<ND>(e, c, p, r, k, evol, S);
+    if (!S.ok()) {
+        double ct[ND + 2], pt[ND + 2];
 #pragma unroll
-            for (int v = 0; v < ND + 2; ++v) {
-                ct[v] = c[v];
-            }
-            to_prim_slow<ND>(e, ct, pt);
+        for (int v = 0; v < ND + 2; ++v) {
+            ct[v] = c[v];
+        }
+        if (e.kind == EOS_PERFECT_GAS_FAST) {
+            to_prim_slow<ND, EOS_PERFECT_GAS_FAST>(e, ct, pt);
+        } else {
+            to_prim_slow<ND, EOS_PERFECT_GAS>(e, ct, pt);
+        }
 #pragma unroll
-            for (int v = 0; v < ND + 2; ++v) {
-                p[v] = pt[v];
-            }
+        for (int v = 0; v < ND + 2; ++v) {
+            p[v] = pt[v];
         }
     }
 }
@@ -552,13 +557,6 @@ __device__ __forceinline__ void to_cons(const Eos& e, const double* p, double* c
     double f[ND + 2];
     to_cons_flux<ND>(e, p, 0, c, f);
 }
-template <int ND>
-__device__ __forceinline__ void flux_prim(const Eos& e, const double* p, int l, double* f)
-{
-    double c[ND + 2];
-    to_cons_flux<ND>(e, p, l, c, f);
-}
-
 __device__ __forceinline__ double sound(const Eos& e, double rho, double P)
 {
     if (e.kind == EOS_RAD_GAS) {
@@ -572,9 +570,22 @@ __device__ __forceinline__ double sound(const Eos& e, double rho, double P)
 
 // What the health check and the CFL need of a new state: the internal energy
 // (main.cpp:397-425), the primitives and the sound speed (time_step.hpp:55-77).
-template <int ND>
+template <int ND, bool TINY = false>
+__device__ __forceinline__ bool state_core(const Eos& e, const double* q, double& evol, double& snd, double* p)
+{
+    q64::Den r, k;
+    q64::Range S(e.consts_ok);
+    prim_core<ND, TINY>(e, q, p, r, k, evol, S);
+    snd = q64::root(q64::quo(e.gamma * p[1 + ND], r));
+    return TINY ? S.dens_ok() : S.ok();
+}
+template <int ND, int KIND>
 static __device__ __noinline__ void state_prims_slow(Eos e, const double* q, double* out)
 {
+    e.kind = KIND;
+    if (e.kind != EOS_RAD_GAS && state_core<ND, true>(e, q, out[0], out[1], out + 2)) {
+        return;
+    }
     out[0] = q[1 + ND] - plain::ek_cons<ND>(q);
     plain::to_prim<ND>(e, q, out + 2);
     out[1] = plain_sound(e, out[2], out[3 + ND]);
@@ -582,23 +593,19 @@ static __device__ __noinline__ void state_prims_slow(Eos e, const double* q, dou
 template <int ND>
 __device__ __forceinline__ void state_prims(const Eos& e, const double* q, double& evol, double& snd, double* p)
 {
-    bool slow = e.kind == EOS_RAD_GAS;
-    if (e.kind != EOS_RAD_GAS) {
-        q64::Den r, k;
-        q64::Range S(e.consts_ok), Z;
-        prim_core<ND>(e, q, p, r, k, evol, S, Z);
-        snd = q64::root(q64::quo(e.gamma * p[1 + ND], r));
-        if (!(S.ok() && Z.ok())) {
-            slow = !(S.ok() && prim_zeros<ND>(e, q));
-        }
-    }
-    if (slow) {
+    if (e.kind == EOS_RAD_GAS || !state_core<ND>(e, q, evol, snd, p)) {
         double qt[ND + 2], ot[ND + 4];
 #pragma unroll
         for (int v = 0; v < ND + 2; ++v) {
             qt[v] = q[v];
         }
-        state_prims_slow<ND>(e, qt, ot);
+        if (e.kind == EOS_PERFECT_GAS_FAST) {
+            state_prims_slow<ND, EOS_PERFECT_GAS_FAST>(e, qt, ot);
+        } else if (e.kind == EOS_RAD_GAS) {
+            state_prims_slow<ND, EOS_RAD_GAS>(e, qt, ot);
+        } else {
+            state_prims_slow<ND, EOS_PERFECT_GAS>(e, qt, ot);
+        }
         evol = ot[0];
         snd = ot[1];
 #pragma unroll
@@ -617,17 +624,17 @@ __device__ __forceinline__ double limited_width(double dl)
 {
     return LIM == LIM_VANLEER ? dl : dl / 2;
 }
-// Z holds the quotients and the limiter's own denominator: in range wherever
-// both quotients are normal-sized, so what is left to the one-by-one look
-// (limited_ok) is flat or extreme data.
+// S holds the quotients and the limiter's own denominator where their product
+// is positive (or not a number): elsewhere the slope is zero whatever they are.
 template <int LIM>
 __device__ __forceinline__ double limited_den(double ratio)
 {
     return LIM == LIM_VANLEER ? (ratio + 1) * (ratio + 1) : (LIM == LIM_MINMOD ? 1 + ratio : (ratio * ratio) + 1);
 }
 template <int LIM>
-__device__ __forceinline__ double limited_core(double dR, double dL, q64::Range& Z)
+__device__ __forceinline__ double limited_core(double dR, double dL, q64::Range& S)
 {
+    const bool use = !(dL * dR <= 0);
     const double ratio = q64::quo(dR, q64::den(dL));
     const double b = limited_den<LIM>(ratio);
     const double num = LIM == LIM_MINMOD ? fmin(1., ratio) : (dR + dL) * ratio;
@@ -635,23 +642,38 @@ __device__ __forceinline__ double limited_core(double dR, double dL, q64::Range&
     if constexpr (LIM == LIM_MINMOD) {
         s = s * (dL + dR);
     }
-    Z.add(dR, dL);
-    Z.add(b);
-    Z.low(dL);
-    Z.low(b);
-    return dL * dR > 0 ? s : 0.0;
+    S.slope(use, dR, dL, b);
+    S.low(dL);
+    S.low(b);
+    return use ? s : 0.0;
 }
+// The same for quotients down to 2^-1000, tiny pairs scaled by a power of two
+// (the slope scales with them); good turns false beyond that.
 template <int LIM>
-__device__ __forceinline__ bool limited_ok(double dR, double dL)
+__device__ __forceinline__ double limited_tiny(double dR, double dL, bool& good)
 {
-    return !(dL * dR > 0) ||
-           (q64::den_ok(dL) && q64::within(dR) && q64::den_ok(limited_den<LIM>(q64::quo(dR, q64::den(dL)))));
+    const double lo = fmin(fabs(dR), fabs(dL));
+    const double hi = fmax(fabs(dR), fabs(dL));
+    const bool use = !(dL * dR <= 0);
+    const double up = lo < 0x1p-700 ? 0x1p400 : 1.0;
+    const double down = lo < 0x1p-700 ? 0x1p-400 : 1.0;
+    const double R = dR * up, L = dL * up;
+    const double ratio = q64::quo(R, q64::den_any(L));
+    const double b = limited_den<LIM>(ratio);
+    const double num = LIM == LIM_MINMOD ? fmin(1., ratio) : (R + L) * ratio;
+    double s = q64::quo(num, q64::den_any(b));
+    if constexpr (LIM == LIM_MINMOD) {
+        s = s * (L + R);
+    }
+    good = !use || (lo >= 0x1p-1000 && hi <= 0x1p200 && ratio >= 0x1p-1000 && ratio <= 0x1p400);
+    return use ? s * down : 0.0;
 }
 // the raw-difference forms of the fast kind
 template <int LIM>
-__device__ __forceinline__ double limited_fast(double dR, double dL, q64::Range& Z)
+__device__ __forceinline__ double limited_fast(double dR, double dL, q64::Range& S)
 {
     const double prod = dR * dL;
+    const bool use = !(prod <= 0);
     double s;
     if constexpr (LIM == LIM_MINMOD) {
         s = fabs(dR) < fabs(dL) ? dR : dL;
@@ -659,30 +681,42 @@ __device__ __forceinline__ double limited_fast(double dR, double dL, q64::Range&
         const double num = LIM == LIM_VANLEER ? prod : prod * (dR + dL);
         const double b = LIM == LIM_VANLEER ? dR + dL : dR * dR + dL * dL;
         s = q64::quo(num, q64::den(b));
-        Z.add(b);
+        S.num_if(use, b);
     }
-    return prod > 0 ? s : 0.0;
+    return use ? s : 0.0;
 }
 template <int LIM>
 __device__ __forceinline__ bool limited_fast_ok(double dR, double dL)
 {
-    return LIM == LIM_MINMOD || !(dR * dL > 0) ||
-           (q64::within(dR) && q64::within(dL) && q64::within(LIM == LIM_VANLEER ? dR + dL : dR * dR + dL * dL));
+    return LIM == LIM_MINMOD || dR * dL <= 0 || q64::num_ok(LIM == LIM_VANLEER ? dR + dL : dR * dR + dL * dL);
 }
 
 // limited_linear_reconstruction.hpp:46-64 for NV variables of one cell along
 // one dimension: values m, c, p of the cell and its neighbours, the distances
 // hL, hR to them and half the cell's width (raw differences of the fast kind:
 // 1, 1 and 1/2).
-template <int NV>
-static __device__ __noinline__ void faces_slow(int kind, int lim, const double* m, const double* c, const double* p,
-                                               double hL, double hR, double half, double* lo, double* hi)
+// One variable again, whatever its size; h_ok: both distances are in range.
+template <int LIM>
+static __device__ __noinline__ void face_slow(int kind, bool h_ok, double m, double c, double p, q64::Den hL, q64::Den hR,
+                                              double half, double* lo, double* hi)
 {
-    for (int v = 0; v < NV; ++v) {
-        const double s = half * plain::slope(lim, (p[v] - c[v]) / hR, (c[v] - m[v]) / hL, kind);
-        lo[v] = c[v] - s;
-        hi[v] = c[v] + s;
+    const double aR = p - c, aL = c - m;
+    double s;
+    if (kind == EOS_PERFECT_GAS_FAST) {
+        if (h_ok && limited_fast_ok<LIM>(aR * hR.y, aL * hL.y)) {
+            return;
+        }
+        s = half * plain::slope(LIM, aR / hR.b, aL / hL.b, kind);
+    } else {
+        bool good = h_ok, pair;
+        const double R = q64::quo_tiny(aR, hR, good), L = q64::quo_tiny(aL, hL, good);
+        s = (LIM == LIM_VANLEER ? 2 * half : half) * limited_tiny<LIM>(R, L, pair);
+        if (!(good && pair)) {
+            s = half * plain::slope(LIM, aR / hR.b, aL / hL.b);
+        }
     }
+    *lo = c - s;
+    *hi = c + s;
 }
 // ld(k, v): variable v of the cell (k = 1) and its neighbours (0, 2);
 // ld_again(k, v) the same for the rare second look, so that a caller with the
@@ -693,38 +727,24 @@ __device__ __forceinline__ void faces_ld(int kind, const Ld& ld, const LdAgain& 
 {
     const bool fast = kind == EOS_PERFECT_GAS_FAST;
     const double w = LIM == LIM_VANLEER ? 2 * half : half;
-    q64::Range Z;
+    q64::Range S;
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
         const double c = ld(1, v);
         const double R = fast ? (ld(2, v) - c) * hR.y : q64::quo(ld(2, v) - c, hR);
         const double L = fast ? (c - ld(0, v)) * hL.y : q64::quo(c - ld(0, v), hL);
-        const double s = w * (fast ? limited_fast<LIM>(R, L, Z) : limited_core<LIM>(R, L, Z));
+        const double s = w * (fast ? limited_fast<LIM>(R, L, S) : limited_core<LIM>(R, L, S));
         lo[v] = c - s;
         hi[v] = c + s;
     }
-    const bool h_ok = q64::den_ok(hR.b) && q64::den_ok(hL.b);
-    if (!(h_ok && Z.ok())) {
-        double mt[NV], ct[NV], pt[NV];
-        bool ok = h_ok;
+    const bool h_ok = q64::width_ok(hR.b) && q64::width_ok(hL.b);
+    if (!(h_ok && S.ok())) {
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
-            mt[v] = ld_again(0, v);
-            ct[v] = ld_again(1, v);
-            pt[v] = ld_again(2, v);
-            const double aR = pt[v] - ct[v], aL = ct[v] - mt[v];
-            ok = ok && (fast ? limited_fast_ok<LIM>(aR * hR.y, aL * hL.y)
-                             : (q64::within0(aR) && q64::within0(aL) &&
-                                limited_ok<LIM>(q64::quo(aR, hR), q64::quo(aL, hL))));
-        }
-        if (!ok) {
-            double lt[NV], ht[NV];
-            faces_slow<NV>(kind, LIM, mt, ct, pt, hL.b, hR.b, half, lt, ht);
-#pragma unroll
-            for (int v = 0; v < NV; ++v) {
-                lo[v] = lt[v];
-                hi[v] = ht[v];
-            }
+            double lt = lo[v], ht = hi[v];
+            face_slow<LIM>(kind, h_ok, ld_again(0, v), ld_again(1, v), ld_again(2, v), hL, hR, half, &lt, &ht);
+            lo[v] = lt;
+            hi[v] = ht;
         }
     }
 }
@@ -742,7 +762,7 @@ __device__ __forceinline__ void faces_lim(int kind, bool uniform, const double* 
     if (kind == EOS_PERFECT_GAS_FAST && uniform) {
         faces_den<NV, LIM>(kind, m, c, p, q64::Den{1.0, 1.0}, q64::Den{1.0, 1.0}, 0.5, lo, hi);
     } else {
-        faces_den<NV, LIM>(kind, m, c, p, q64::den((dl_m + dl) / 2), q64::den((dl + dl_p) / 2), dl / 2, lo, hi);
+        faces_den<NV, LIM>(kind, m, c, p, q64::den_any((dl_m + dl) / 2), q64::den_any((dl + dl_p) / 2), dl / 2, lo, hi);
     }
 }
 template <int NV>
@@ -765,17 +785,16 @@ __device__ __forceinline__ void faces(int kind, int lim, bool uniform, const dou
 }
 
 // hydro/riemann_solver.hpp:22-134 (HLL and HLLC).  HLLC needs the flux of the
-// side the star state lies on only.  zeros: the operands besides the momenta
-// that may be zero and are.
-template <int ND, int RS>
+// side the star state lies on only.
+template <int ND, int RS, bool TINY = false>
 __device__ __forceinline__ void riemann_core(const Eos& e, const double* cL, const double* cR, int l, double* f,
-                                             q64::Range& S, q64::Range& Z, bool& zeros)
+                                             q64::Range& S)
 {
     constexpr int NV = ND + 2;
     double pL[NV], pR[NV], evL, evR;
     q64::Den rL, rR, kL{}, kR{};
-    prim_core<ND>(e, cL, pL, rL, kL, evL, S, Z);
-    prim_core<ND>(e, cR, pR, rR, kR, evR, S, Z);
+    prim_core<ND, TINY>(e, cL, pL, rL, kL, evL, S);
+    prim_core<ND, TINY>(e, cR, pR, rR, kR, evR, S);
     const double PL = pL[1 + ND], PR = pR[1 + ND];
     const double aL = q64::root(q64::quo(e.gamma * PL, rL));
     const double aR = q64::root(q64::quo(e.gamma * PR, rR));
@@ -801,7 +820,6 @@ __device__ __forceinline__ void riemann_core(const Eos& e, const double* cL, con
         fs[1 + l] += p[1 + ND];
         fs[1 + ND] = p[1 + l] * (E + p[1 + ND]);
     };
-    zeros = true;
     if constexpr (RS == RS_HLL) {
         double fL[NV], fR[NV];
         side_flux(pL, kL, fL);
@@ -813,9 +831,8 @@ __device__ __forceinline__ void riemann_core(const Eos& e, const double* cL, con
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
             const double num = (nR * fL[v]) - (nL * fR[v]) + (nL * nR * (cR[v] - cL[v]));
-            f[v] = q64::quo(num, w);
-            Z.add(num);
-            zeros = zeros && q64::within0(num);
+            f[v] = num_quo<TINY>(num, w, S);
+            S.num(num, num);
         }
     } else {
         const double rcL = pL[0] * (wsL - uL);
@@ -823,7 +840,7 @@ __device__ __forceinline__ void riemann_core(const Eos& e, const double* cL, con
         const double un_num = PR - PL + (rcL * uL) - (rcR * uR);
         // rcL - rcR < 0: quo keeps a zero's sign for positive denominators
         const q64::Den du = q64::den(-(rcL - rcR));
-        const double ustar = -q64::quo(un_num, du);
+        const double ustar = -num_quo<TINY>(un_num, du, S);
         const double pstar = 1. / 2 * (PL + PR + (rcL * (ustar - uL)) + (rcR * (ustar - uR)));
         const bool left = ustar > 0;
         const double Sw = left ? wsL : wsR;
@@ -841,8 +858,9 @@ __device__ __forceinline__ void riemann_core(const Eos& e, const double* cL, con
         S.den(du.b);
         S.den(su.b);
         S.add(sn);
-        Z.add(un_num, un_s);
-        zeros = q64::within0(un_num) && q64::within0(un_s);
+        if (e.kind != EOS_PERFECT_GAS_FAST) {
+            S.num(un_num, un_s);
+        }
         double rs, Es;
         if (e.kind == EOS_PERFECT_GAS_FAST) {
             const double ratio = sn * su.y;
@@ -850,7 +868,7 @@ __device__ __forceinline__ void riemann_core(const Eos& e, const double* cL, con
             Es = ratio * cs[1 + ND] + un_s * su.y * (ustar * cs[0] * sn + ps[1 + ND]);
         } else {
             rs = q64::quo(cs[0] * sn, su);
-            Es = (q64::quo(sn, su) * cs[1 + ND]) + (q64::quo(un_s, su) * ((ustar * cs[0] * sn) + ps[1 + ND]));
+            Es = (q64::quo(sn, su) * cs[1 + ND]) + (num_quo<TINY>(un_s, su, S) * ((ustar * cs[0] * sn) + ps[1 + ND]));
         }
         const double rsu = rs * ustar;
         const bool sup = wsL * wsR > 0;
@@ -868,25 +886,36 @@ __device__ __forceinline__ void riemann_core(const Eos& e, const double* cL, con
     }
 }
 
+template <int ND, int RS, int KIND>
+static __device__ __noinline__ void riemann_slow(Eos e, const double* cL, const double* cR, int l, double* f)
+{
+    e.kind = KIND;
+    q64::Range S(e.consts_ok);
+    riemann_core<ND, RS, true>(e, cL, cR, l, f, S);
+    if (!S.dens_ok()) {
+        plain::riemann<ND>(e, RS, cL, cR, l, f);
+    }
+}
 template <int ND, int RS>
 __device__ __forceinline__ void riemann_rs(const Eos& e, const double* cL, const double* cR, int l, double* f)
 {
-    q64::Range S(e.consts_ok), Z;
-    bool zeros;
-    riemann_core<ND, RS>(e, cL, cR, l, f, S, Z, zeros);
-    if (!(S.ok() && Z.ok())) {
-        if (!(S.ok() && zeros && prim_zeros<ND>(e, cL) && prim_zeros<ND>(e, cR))) {
-            double lt[ND + 2], rt[ND + 2], ft[ND + 2];
+    q64::Range S(e.consts_ok);
+    riemann_core<ND, RS>(e, cL, cR, l, f, S);
+    if (!S.ok()) {
+        double lt[ND + 2], rt[ND + 2], ft[ND + 2];
 #pragma unroll
-            for (int v = 0; v < ND + 2; ++v) {
-                lt[v] = cL[v];
-                rt[v] = cR[v];
-            }
-            riemann_slow<ND>(e, RS, lt, rt, l, ft);
+        for (int v = 0; v < ND + 2; ++v) {
+            lt[v] = cL[v];
+            rt[v] = cR[v];
+        }
+        if (e.kind == EOS_PERFECT_GAS_FAST) {
+            riemann_slow<ND, RS, EOS_PERFECT_GAS_FAST>(e, lt, rt, l, ft);
+        } else {
+            riemann_slow<ND, RS, EOS_PERFECT_GAS>(e, lt, rt, l, ft);
+        }
 #pragma unroll
-            for (int v = 0; v < ND + 2; ++v) {
-                f[v] = ft[v];
-            }
+        for (int v = 0; v < ND + 2; ++v) {
+            f[v] = ft[v];
         }
     }
 }

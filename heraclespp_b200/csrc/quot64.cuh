@@ -17,8 +17,8 @@
 // the rounded reciprocal of b and q0 = RN(a y), RN(q0 + y RN(a - b q0)) is the
 // rounded quotient.  The square root is the same scheme on the reciprocal
 // square root.  Both need operands far from overflow and underflow: callers
-// gather a group's operands in a Range and fall back to the plain operators
-// for the whole group when one lies outside (numerators may be zero).
+// gather a group's operands in a Range and take the plain operators where one
+// lies outside.
 // tests/test_gpu_quot64.py holds the functions built on them to the CPU's
 // operators, bit for bit, over all exponents.
 #pragma once
@@ -27,10 +27,20 @@
 
 namespace hcl::q64 {
 
-// Operands of a group must lie within 2^+-300: quotients then stay within
-// 2^+-600 (squares and products of two within 2^+-900) and a residual, 2^-106
-// of its numerator at the least, stays normal.
+// Denominators and pressures of a group must lie within 2^-300 and 2^200.
 constexpr int kExp = 300;
+constexpr int kTopExp = 200;
+// Numerators (momenta, differences, the two quotients of a slope) may be as
+// small as 2^-800: a quotient then stays above 2^-1000 and a residual, 2^-106
+// of its numerator at the least, above 2^-906.  A kinetic energy whose own
+// numerator (the squared momentum) is too small for a right residual, below
+// 2^-916, is below 2^-616 itself and vanishes next to an internal energy of
+// 2^-310 under either rounding.  Gas at rest ahead of a front needs the range:
+// there velocities fall by orders of magnitude per cell, down to exact zeros.
+constexpr int kNumExp = 800;
+// A one-sided quotient is a difference over a width: from 2^-116 up, a quotient
+// above 2^-800 had a difference above 2^-916.
+constexpr int kWidthExp = 116;
 
 // The high word of a double read as a float orders like the double's
 // magnitude (sign, the upper eight exponent bits, then the rest); infinities
@@ -45,7 +55,21 @@ __device__ __forceinline__ float lo_bound()
 }
 __device__ __forceinline__ float hi_bound()
 {
-    return __int_as_float((1023 + kExp) << 20);
+    return __int_as_float((1023 + kTopExp) << 20);
+}
+__device__ __forceinline__ float num_bound()
+{
+    return __int_as_float((1023 - kNumExp) << 20);
+}
+__device__ __forceinline__ bool nonzero(double a)
+{
+    return ((__double2hiint(a) & 0x7fffffff) | __double2loint(a)) != 0;
+}
+// a numerator that quo() may take: zero, or of the size above
+__device__ __forceinline__ bool num_ok(double a)
+{
+    const float f = fabsf(hi_float(a));
+    return !nonzero(a) || (f >= num_bound() && f <= hi_bound());
 }
 __device__ __forceinline__ bool within(double a)
 {
@@ -58,19 +82,28 @@ __device__ __forceinline__ bool within0(double a)
 }
 // The reciprocal iteration stops one unit short where the significand of b is
 // all ones (the theorem's known exception: 1 / (2 - 2^-52) lies next to a
-// midpoint); a low word of ones sends those to the plain operators.
+// midpoint); a low word of ones sends those to the plain operators, except
+// where such a denominator is an ordinary one (den_any).
 __device__ __forceinline__ bool den_ok(double b)
 {
     return within(b) && __double2loint(b) != -1;
 }
 
+// of a width whose Den comes from den_any() or a division
+__device__ __forceinline__ bool width_ok(double b)
+{
+    return within(b) && fabsf(hi_float(b)) >= __int_as_float((1023 - kWidthExp) << 20);
+}
+
 // The operands of a group, gathered at half an instruction per bound and
-// operand (three-input minimum and maximum, NaN-propagating).
+// operand (three-input minimum and maximum, NaN-propagating); numerators, which
+// may be zero, at two and a half.
 struct Range {
     float mn, mx;
+    float nz;      // smallest numerator besides zeros
     unsigned ones; // largest low word of the denominators
 
-    __device__ __forceinline__ explicit Range(bool good = true) : mn(good ? 1.f : 0.f), mx(1.f), ones(0u) {}
+    __device__ __forceinline__ explicit Range(bool good = true) : mn(good ? 1.f : 0.f), mx(1.f), nz(1.f), ones(0u) {}
     __device__ __forceinline__ void add(double a)
     {
         const float f = fabsf(hi_float(a));
@@ -81,7 +114,44 @@ struct Range {
     {
         const float f = fabsf(hi_float(a)), g = fabsf(hi_float(b));
         asm("min.NaN.f32 %0, %0, %1, %2;" : "+f"(mn) : "f"(f), "f"(g));
+        top(a, b);
+    }
+    __device__ __forceinline__ void top(double a, double b)
+    {
+        const float f = fabsf(hi_float(a)), g = fabsf(hi_float(b));
         asm("max.NaN.f32 %0, %0, %1, %2;" : "+f"(mx) : "f"(f), "f"(g));
+    }
+    // numerators
+    __device__ __forceinline__ void num(double a, double b)
+    {
+        top(a, b);
+        low_num(a);
+        low_num(b);
+    }
+    __device__ __forceinline__ void low_num(double a)
+    {
+        if (nonzero(a)) {
+            asm("min.f32 %0, %0, %1;" : "+f"(nz) : "f"(fabsf(hi_float(a))));
+        }
+    }
+    // the two quotients of a slope and the upper bound of its own denominator
+    // (at least one), where the slope is not zero
+    __device__ __forceinline__ void slope(bool use, double r, double l, double b)
+    {
+        const float f = fabsf(hi_float(r)), g = fabsf(hi_float(l)), h = fabsf(hi_float(b));
+        top(r, l);
+        if (use) {
+            asm("min.f32 %0, %0, %1, %2;" : "+f"(nz) : "f"(f), "f"(g));
+            asm("max.NaN.f32 %0, %0, %1;" : "+f"(mx) : "f"(h));
+        }
+    }
+    // such a denominator where nothing else is of concern
+    __device__ __forceinline__ void num_if(bool use, double b)
+    {
+        if (use) {
+            asm("min.f32 %0, %0, %1;" : "+f"(nz) : "f"(fabsf(hi_float(b))));
+            asm("max.NaN.f32 %0, %0, %1;" : "+f"(mx) : "f"(fabsf(hi_float(b))));
+        }
     }
     // low words of denominators added elsewhere
     __device__ __forceinline__ void low(double b)
@@ -93,9 +163,19 @@ struct Range {
         add(b);
         low(b);
     }
-    __device__ __forceinline__ bool ok() const
+    // what was found unfit elsewhere
+    __device__ __forceinline__ void also(bool good)
+    {
+        mn = good ? mn : 0.f;
+    }
+    // all but the numerators' lower bound
+    __device__ __forceinline__ bool dens_ok() const
     {
         return mn >= lo_bound() && mx <= hi_bound() && ones != 0xffffffffu;
+    }
+    __device__ __forceinline__ bool ok() const
+    {
+        return dens_ok() && nz >= num_bound();
     }
 };
 
@@ -115,12 +195,34 @@ __device__ __forceinline__ Den den(double b)
     y = __fma_rn(y, __fma_rn(-b, y, 1.0), y);
     return den_from(b, y);
 }
+// the same for a denominator whose significand may well be all ones: the density
+// next to 1 of a gas at rest, a width next to a power of two.  There the
+// second step's correction, 2^-54, is a tie short of the true 2^-54 + 2^-107; one
+// unit of its last place carries it past.
+__device__ __forceinline__ Den den_any(double b)
+{
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    y = __fma_rn(y, __fma_rn(-b, y, 1.0), y);
+    const double e = __fma_rn(-b, y, 1.0);
+    return Den{b, __fma_rn(y, __fma_rn(e, 0x1p-52, e), y)};
+}
 // a / d.b; the residual is formed as b q0 - a so that a zero numerator keeps
 // its sign (d.b > 0)
 __device__ __forceinline__ double quo(double a, const Den& d)
 {
     const double q = __dmul_rn(a, d.y);
     return __fma_rn(-__fma_rn(d.b, q, -a), d.y, q);
+}
+
+// the same for a numerator down to the smallest, scaled by a power of two; good
+// turns false where the scaling back would round again
+__device__ __forceinline__ double quo_tiny(double a, const Den& d, bool& good)
+{
+    const bool up = fabs(a) < 0x1p-700;
+    const double q = quo(a * (up ? 0x1p300 : 1.0), d) * (up ? 0x1p-300 : 1.0);
+    good = good && (!nonzero(a) || fabs(q) >= 0x1p-1021);
+    return q;
 }
 
 __device__ __forceinline__ double root(double x)
