@@ -456,29 +456,37 @@ int march3d64_configure_t()
     });
 }
 
+// How `sms` SMs, one CTA each, cover the grid: the planes per CTA with the fewest
+// plane steps over all waves (a CTA repeats two planes of face states and stages
+// two more), and that count.
+struct M3Plan {
+    int ntx, nty, L;
+    int64_t cost;
+};
+inline M3Plan march3d64_plan(const GridDev& g, int sms)
+{
+    M3Plan p{(g.nx[0] + kM3X - 1) / kM3X, (g.nx[1] + kM3Y - 1) / kM3Y, g.nx[2], INT64_MAX};
+    const int64_t nt = (int64_t)p.ntx * p.nty;
+    for (int c = 1; c <= g.nx[2]; ++c) {
+        const int L = (g.nx[2] + c - 1) / c;
+        const int64_t ctas = nt * ((g.nx[2] + L - 1) / L);
+        const int64_t cost = ((ctas + sms - 1) / sms) * (L + 3);
+        if (cost < p.cost) {
+            p.cost = cost;
+            p.L = L;
+        }
+    }
+    return p;
+}
+
 template <int LIM, int RS, int KIND>
 void march3d64_launch_t(const GridDev& g, const StateDev& in, const StateDev& out, StepCtl* ctl, const RunParamsDev& rp,
                         int slot, int out_buf, cudaStream_t s)
 {
     const int sms = march3d64_configure_t<LIM, RS, KIND>();
-    const int ntx = (g.nx[0] + kM3X - 1) / kM3X;
-    const int nty = (g.nx[1] + kM3Y - 1) / kM3Y;
-    const int nt = ntx * nty;
-    // planes per CTA: the fewest plane steps over all waves (a CTA repeats two
-    // planes of face states and stages two more)
-    int best_L = g.nx[2];
-    int64_t best = INT64_MAX;
-    for (int c = 1; c <= g.nx[2]; ++c) {
-        const int L = (g.nx[2] + c - 1) / c;
-        const int64_t ctas = (int64_t)nt * ((g.nx[2] + L - 1) / L);
-        const int64_t cost = ((ctas + sms - 1) / sms) * (L + 3);
-        if (cost < best) {
-            best = cost;
-            best_L = L;
-        }
-    }
-    const int blocks = nt * ((g.nx[2] + best_L - 1) / best_L);
-    k_march3d64<LIM, RS, KIND><<<blocks, kM3T, sizeof(M3Shared), s>>>(g, in, out, ctl, rp, slot, out_buf, ntx, nty, best_L);
+    const M3Plan p = march3d64_plan(g, sms);
+    const int blocks = p.ntx * p.nty * ((g.nx[2] + p.L - 1) / p.L);
+    k_march3d64<LIM, RS, KIND><<<blocks, kM3T, sizeof(M3Shared), s>>>(g, in, out, ctl, rp, slot, out_buf, p.ntx, p.nty, p.L);
     ++g_launches;
 }
 

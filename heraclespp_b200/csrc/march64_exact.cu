@@ -17,6 +17,18 @@ bool march1d64_valid(const GridDev& g)
            march1d64_configure_t<EOS_PERFECT_GAS>();
 }
 
+static int sm_count()
+{
+    static PerDevice cache;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    return cache.get(dev, [dev] {
+        int v = 0;
+        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+        return v;
+    });
+}
+
 // Cartesian 2-D grids of the perfect gas without scalars or pressure fix, from
 // more 16 x 16 tiles than one wave of the tile kernel holds (two per SM): a
 // strip is at least four row iterations deep, a single tile is quicker (us per
@@ -24,22 +36,26 @@ bool march1d64_valid(const GridDev& g)
 // 59.7 and 45.6)
 bool march2d64_valid(const GridDev& g)
 {
-    static PerDevice cache;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    const int sms = cache.get(dev, [dev] {
-        int v = 0;
-        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-        return v;
-    });
+    const int sms = sm_count();
     return g.ndim == 2 && g.geom == GEOM_CARTESIAN && g.eos == EOS_PERFECT_GAS && g.nfx == 0 && !g.pressure_fix &&
            (int64_t)((g.nx[0] + 15) / 16) * ((g.nx[1] + 15) / 16) > 2 * sms;
 }
 
-// Cartesian 3-D grids, the same
+// Cartesian 3-D grids, the same, where the march's plane steps take less than the
+// waves of 8 x 8 x 4 tiles (one per SM): 10.3 us each less 4 against 17.2 us each
+// and 6 (in the fast forms 8.0 and 13.2).  A CTA marches at least three planes of
+// 30 x 10 columns, so small grids are quicker as tiles (us per step, tile and
+// march: 32^3 24 and 50, 48^3 60 and 70, 64^3 126 and 142, 56^3 92 and 80, 80^3 240
+// and 183, 128^3 932 and 776, 200 x 100 x 4 61 and 47).
 bool march3d64_valid(const GridDev& g)
 {
-    return g.ndim == 3 && g.geom == GEOM_CARTESIAN && g.eos == EOS_PERFECT_GAS && g.nfx == 0 && !g.pressure_fix;
+    if (g.ndim != 3 || g.geom != GEOM_CARTESIAN || g.eos != EOS_PERFECT_GAS || g.nfx != 0 || g.pressure_fix) {
+        return false;
+    }
+    const int sms = sm_count();
+    const int64_t tiles = (int64_t)((g.nx[0] + 7) / 8) * ((g.nx[1] + 7) / 8) * ((g.nx[2] + 3) / 4);
+    const int64_t waves = (tiles + sms - 1) / sms;
+    return 5 * waves + 3 > 3 * march3d64_plan(g, sms).cost;
 }
 
 void configure_march_exact(const GridDev& g)
