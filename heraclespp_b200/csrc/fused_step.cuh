@@ -358,17 +358,20 @@ __device__ __forceinline__ void store_images_3d(double* __restrict__ q, int64_t 
 // more resident CTAs fill those waits.  Where the shared memory of a launch
 // leaves room for them the 2-D FP64 tile runs two CTAs per SM (128 registers,
 // some spilled; KH 2048^2 with a passive scalar 1.75 ms per step unbounded,
-// 1.10 ms so).  The straight-line quotients hold more values at once than the
+// 0.99 ms so).  The straight-line quotients hold more values at once than the
 // branching divisions did: three CTAs (80 registers) spill 1.5 KB per thread.
+// RadGas still divides with a branch and waits more: three CTAs (1024^2, Minmod
+// and HLLC: 2.20 ms per step, two CTAs 2.69; 256^2, two tiles per SM, 213 and 202
+// us).
 // The other tiles (0 here) keep the compiler's register choice: the 3-D FP64
 // tile at one CTA and 255 registers measures as at two and 128 (a spherical
 // 96 x 64 x 50 step 0.22 ms), and asking for a minimum of one block lets the
 // FP32-mixed 3-D tile take too many registers (RT 256^2 x 512 with a passive
 // scalar 8.8 -> 14.3 ms).
-template <int ND, bool EXACT, int TX, int TY, int TZ>
+template <int ND, bool EXACT, int EOSK>
 constexpr int fused_min_blocks()
 {
-    return (EXACT && ND == 2) ? 2 : 0;
+    return (EXACT && ND == 2) ? (EOSK == EOS_RAD_GAS ? 3 : 2) : 0;
 }
 
 // tma (2-D and 3-D): the FP64 tile plus its halo arrives as one tensor box
@@ -1460,7 +1463,7 @@ k_fused_step_wide(GridDev g, StateDev in, StateDev out, StepCtl* ctl, RunParamsD
 // the same step with the occupancy bound above (instantiated where it is > 0)
 template <int ND, bool EXACT, int TX, int TY, int TZ, int EOSK = EOS_PERFECT_GAS>
 __global__ void __launch_bounds__(TX*(ND >= 2 ? TY : 1)*(ND >= 3 ? TZ : 1),
-                                  fused_min_blocks<ND, EXACT, TX, TY, TZ>() > 0 ? fused_min_blocks<ND, EXACT, TX, TY, TZ>() : 1)
+                                  fused_min_blocks<ND, EXACT, EOSK>() > 0 ? fused_min_blocks<ND, EXACT, EOSK>() : 1)
 k_fused_step_occ(GridDev g, StateDev in, StateDev out, StepCtl* ctl, RunParamsDev rp, int slot, int out_buf,
                  const __grid_constant__ CUtensorMap tmap, int tma)
 {
@@ -1483,7 +1486,7 @@ struct FusedLauncher {
     // block (launches without passive scalars use smem(0) and keep their
     // occupancy); called once per process before any launch (never during
     // stream capture).
-    static constexpr int kMinBlocks = fused_min_blocks<ND, EXACT, TX, TY, TZ>();
+    static constexpr bool kBounded = fused_min_blocks<ND, EXACT, EOS_PERFECT_GAS>() > 0;
     static constexpr bool kWide = ND == 2 && TX == 16 && TY == 16;
     template <int EOSK>
     static void configure_wide()
@@ -1499,7 +1502,7 @@ struct FusedLauncher {
         if constexpr (EXACT) {
             set_max_dynamic(reinterpret_cast<const void*>(k_fused_step<ND, EXACT, TX, TY, TZ, EOS_RAD_GAS>));
         }
-        if constexpr (kMinBlocks > 0) {
+        if constexpr (kBounded) {
             set_max_dynamic(reinterpret_cast<const void*>(k_fused_step_occ<ND, EXACT, TX, TY, TZ>));
             if constexpr (EXACT) {
                 set_max_dynamic(reinterpret_cast<const void*>(k_fused_step_occ<ND, EXACT, TX, TY, TZ, EOS_RAD_GAS>));
@@ -1519,9 +1522,10 @@ struct FusedLauncher {
     }
     // the occupancy-bounded kernel pays off when that many CTAs fit the SM's
     // shared memory (1 KB reserved per CTA, up to 512 B static)
+    template <int EOSK>
     static bool use_occ(int nfx)
     {
-        if constexpr (kMinBlocks > 0) {
+        if constexpr (kBounded) {
             static PerDevice cache;
             int dev = 0;
             cudaGetDevice(&dev);
@@ -1530,7 +1534,7 @@ struct FusedLauncher {
                 cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
                 return v;
             });
-            return (size_t)kMinBlocks * (smem(nfx) + 1024 + 512) <= (size_t)per_sm;
+            return (size_t)fused_min_blocks<ND, EXACT, EOSK>() * (smem(nfx) + 1024 + 512) <= (size_t)per_sm;
         }
         return false;
     }
@@ -1570,7 +1574,7 @@ struct FusedLauncher {
                 return;
             }
         }
-        if (use_occ(g.nfx)) {
+        if (use_occ<EOSK>(g.nfx)) {
             k_fused_step_occ<ND, EXACT, TX, TY, TZ, EOSK>
                 <<<blocks, S::TVOL, sm, s>>>(g, in, out, ctl, rp, slot, out_buf, map, tma);
         } else {
@@ -1596,7 +1600,7 @@ struct FusedLauncher {
         static_assert(EXACT, "fast FP64 runs the FP64 kernels");
         configure_wide<EOS_PERFECT_GAS_FAST>();
         set_max_dynamic(reinterpret_cast<const void*>(k_fused_step<ND, EXACT, TX, TY, TZ, EOS_PERFECT_GAS_FAST>));
-        if constexpr (kMinBlocks > 0) {
+        if constexpr (kBounded) {
             set_max_dynamic(reinterpret_cast<const void*>(k_fused_step_occ<ND, EXACT, TX, TY, TZ, EOS_PERFECT_GAS_FAST>));
         }
     }
