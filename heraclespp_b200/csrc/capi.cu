@@ -1610,7 +1610,8 @@ int hcl_run(hcl_handle* h, const hcl_run_params* p, hcl_run_result* r)
                                  h->stream));
         rp.dts = h->d_dts;
     }
-    if (h->cfg.precision != HCL_FP32_MIXED && hcl::fused::march1d64_valid(h->g)) {
+    if ((h->cfg.precision == HCL_FP64 && hcl::fused::march1d_exact_valid(h->g)) ||
+        (h->cfg.precision == HCL_FP64_FAST && hcl::fused::march1d_fast_valid(h->g))) {
         // one launch carries many steps and ends early when the run stops
         constexpr int kMaxSteps = 4096;
         for (int done = 0;;) {

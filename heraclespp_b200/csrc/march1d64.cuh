@@ -446,6 +446,16 @@ bool march1d64_configure_t()
     }) != 0;
 }
 
+// Perfect-gas 1-D domains without scalars or pressure fix, with a gravity table
+// that does not change from step to step, up to 16 CTAs' cells, where this kind's
+// kernel can be launched
+template <int KIND>
+bool march1d64_valid_t(const GridDev& g)
+{
+    return g.ndim == 1 && g.eos == EOS_PERFECT_GAS && g.nfx == 0 && !g.pressure_fix &&
+           g.gravity != GRAV_INTERNAL_MASS && g.nx[0] <= kM1MaxCtas * kM1MaxChunk && march1d64_configure_t<KIND>();
+}
+
 // cells per CTA: the smallest multiple of 32 that 16 CTAs cover the domain with
 inline int march1d64_chunk(const GridDev& g)
 {

@@ -8,13 +8,9 @@
 
 namespace hcl::fused {
 
-// Perfect-gas 1-D domains without scalars or pressure fix, with a gravity
-// table that does not change from step to step, up to 16 CTAs' cells
-bool march1d64_valid(const GridDev& g)
+bool march1d_exact_valid(const GridDev& g)
 {
-    return g.ndim == 1 && g.eos == EOS_PERFECT_GAS && g.nfx == 0 && !g.pressure_fix &&
-           g.gravity != GRAV_INTERNAL_MASS && g.nx[0] <= kM1MaxCtas * kM1MaxChunk &&
-           march1d64_configure_t<EOS_PERFECT_GAS>();
+    return march1d64_valid_t<EOS_PERFECT_GAS>(g);
 }
 
 static int sm_count()

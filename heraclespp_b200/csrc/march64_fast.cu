@@ -8,6 +8,11 @@
 
 namespace hcl::fused {
 
+bool march1d_fast_valid(const GridDev& g)
+{
+    return march1d64_valid_t<EOS_PERFECT_GAS_FAST>(g);
+}
+
 void configure_march_fast(const GridDev& g)
 {
     if (g.ndim == 1) {

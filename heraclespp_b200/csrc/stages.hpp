@@ -115,15 +115,18 @@ bool strip2d_tma_eligible(const GridDev& g);
 // stride is not a multiple of 16 bytes.
 bool encode_tile_map(const GridDev& g, const StateDev& st, int nv, const int box[3], CUtensorMap* map);
 void configure_exact();
-// FP64 march kernels (march64_exact.cu, march64_fast.cu): the step of the
-// grids march2d64_valid() accepts, and their once-per-device set-up
+// FP64 march kernels (march64_exact.cu, march64_fast.cu).
 // 1-D domains that one cluster steps on its own, many steps per launch
-// (march1d64.cuh): `steps` steps from the state of step counter slot0 % 6
-bool march1d64_valid(const GridDev& g);
+// (march1d64.cuh): `steps` steps from the state of step counter slot0 % 6, of the
+// domains for which that kind's kernel fits the device
+bool march1d_exact_valid(const GridDev& g);
+bool march1d_fast_valid(const GridDev& g);
 void march1d_exact(const GridDev& g, const StateDev& st0, const StateDev& st1, StepCtl* ctl, const RunParamsDev& rp,
                    int slot0, int steps, cudaStream_t s);
 void march1d_fast(const GridDev& g, const StateDev& st0, const StateDev& st1, StepCtl* ctl, const RunParamsDev& rp,
                   int slot0, int steps, cudaStream_t s);
+// 2-D and 3-D: the step of the grids march2d64_valid() and march3d64_valid()
+// accept, and their once-per-device set-up
 bool march2d64_valid(const GridDev& g);
 bool march3d64_valid(const GridDev& g);
 void configure_march_exact(const GridDev& g);
