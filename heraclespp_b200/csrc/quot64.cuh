@@ -14,13 +14,25 @@
 // Method: Newton's iteration on the hardware's reciprocal approximation, then
 // the residual correction of Markstein (IBM J. Res. Dev. 34, 1990; Cornea,
 // Harrison and Tang, "Scientific Computing on Itanium", 2002, ch. 4): with y
-// the rounded reciprocal of b and q0 = RN(a y), RN(q0 + y RN(a - b q0)) is the
-// rounded quotient.  The square root is the same scheme on the reciprocal
-// square root.  Both need operands far from overflow and underflow: callers
-// gather a group's operands in a Range and take the plain operators where one
-// lies outside.
-// tests/test_gpu_quot64.py holds the functions built on them to the CPU's
-// operators, bit for bit, over all exponents.
+// the reciprocal of b and q0 = RN(a y), RN(q0 + y RN(a - b q0)) is the rounded
+// quotient.  The square root is the same scheme on the reciprocal square root.
+// Both need operands far from overflow and underflow: callers gather a group's
+// operands in a Range and take the plain operators where one lies outside.
+//
+// What the quotient rests on.  The theorem wants the rounded reciprocal.  Two
+// quadratic steps from a seed good to 2^-19 or better leave 2^-76, so about one
+// y in 2^22 lies on the wrong side of a midpoint.  The quotient is still the
+// rounded one unless |1 - b y| exceeds 2^-52 / b (b scaled to [1, 2); a quotient
+// that is no midpoint is 2^-53 / b of a unit or more away from one): with y off by
+// half a unit and 2^-76 that takes b > 2 (1 - 2^-23).  Those denominators share
+// their high word, and with it the seed, which is one half exactly: for
+// b = 2 - k 2^-52 the first step gives 1/2 + k 2^-54 rounded, and the second the
+// rounded reciprocal for all k (1/b lies k^2 2^-107 past a midpoint for odd k, the
+// step falls 2^-107 short of 1/b) but one: k = 1.  tests/test_gpu_extreme_operands.py
+// divides by all odd k to 2^14 the numerators whose quotients lie next to a
+// midpoint, and takes every stage entry point through extreme operands;
+// tests/test_gpu_quot64.py converts states over all exponents, bit for bit
+// against the CPU's operators.
 #pragma once
 
 #include <cstdint>
@@ -80,9 +92,8 @@ __device__ __forceinline__ bool within0(double a)
 {
     return within(a) || a == 0.0;
 }
-// The reciprocal iteration stops one unit short where the significand of b is
-// all ones (the theorem's known exception: 1 / (2 - 2^-52) lies next to a
-// midpoint); a low word of ones sends those to the plain operators, except
+// The reciprocal stops one unit short where the significand of b is all ones
+// (k = 1 above); a low word of ones sends those to the plain operators, except
 // where such a denominator is an ordinary one (den_any).
 __device__ __forceinline__ bool den_ok(double b)
 {
