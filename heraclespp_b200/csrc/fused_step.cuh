@@ -1332,8 +1332,12 @@ __device__ __forceinline__ void fused_step_body(const GridDev& g, const StateDev
 #pragma unroll
                         for (int d = 0; d < ND; ++d) {
                             const double a = inv_rho_u[d] + sound;
-                            const q64::Den w = q64::den(dxg[d]);
-                            cell += EXACT && q64::within(a) && q64::den_ok(w.b) ? q64::quo(a, w) : a / w.b;
+                            if constexpr (EXACT) {
+                                const q64::Den w = q64::den(dxg[d]);
+                                cell += q64::within(a) && q64::den_ok(w.b) ? q64::quo(a, w) : a / w.b;
+                            } else {
+                                cell += a / dxg[d];
+                            }
                         }
                     }
                     if (isnan(cell)) {

@@ -113,13 +113,13 @@ __device__ __forceinline__ q64::Den face_width(bool unif, double dl, double dl_p
     return FAST ? q64::Den{h, 1.0 / h} : q64::den_any(h);
 }
 
-template <int LIM, int RS, int KIND>
-__device__ __forceinline__ void march2d_riemann(const exact::Eos& e, const double* cL, const double* cR, int l, double* f)
+template <int ND, int RS>
+__device__ __forceinline__ void march_riemann(const exact::Eos& e, const double* cL, const double* cR, int l, double* f)
 {
     if constexpr (RS == RS_SPLITTING) {
-        exact::plain::riemann<2>(e, RS, cL, cR, l, f);
+        exact::plain::riemann<ND>(e, RS, cL, cR, l, f);
     } else {
-        exact::riemann_rs<2, RS>(e, cL, cR, l, f);
+        exact::riemann_rs<ND, RS>(e, cL, cR, l, f);
     }
 }
 
@@ -358,7 +358,7 @@ __device__ __forceinline__ void march2d_strip(const GridDev& g, const double* __
         // y-face j-1/2, and row j-1 is complete
         double G[4] = {0.0, 0.0, 0.0, 0.0};
         if (j >= r0) {
-            march2d_riemann<LIM, RS, KIND>(e, hyT, U[2], 1, G);
+            march_riemann<2, RS>(e, hyT, U[2], 1, G);
         }
         if (j > r0) {
             const int r = j - 1;
@@ -422,7 +422,7 @@ __device__ __forceinline__ void march2d_strip(const GridDev& g, const double* __
             for (int v = 0; v < 4; ++v) {
                 uL[v] = __shfl_up_sync(FULL, U[1][v], 1);
             }
-            march2d_riemann<LIM, RS, KIND>(e, uL, U[0], 0, Fl);
+            march_riemann<2, RS>(e, uL, U[0], 0, Fl);
             dtodv1 = 2 * dthv; // dt / dv: dt = 2 dth
 #pragma unroll
             for (int v = 0; v < 4; ++v) {

@@ -56,16 +56,6 @@ struct M3Shared {
 };
 
 template <int LIM, int RS, int KIND>
-__device__ __forceinline__ void march3d_riemann(const exact::Eos& e, const double* cL, const double* cR, int l, double* f)
-{
-    if constexpr (RS == RS_SPLITTING) {
-        exact::plain::riemann<3>(e, RS, cL, cR, l, f);
-    } else {
-        exact::riemann_rs<3, RS>(e, cL, cR, l, f);
-    }
-}
-
-template <int LIM, int RS, int KIND>
 __global__ void __launch_bounds__(kM3T, 1)
 k_march3d64(GridDev g, StateDev in, StateDev out, StepCtl* ctl, RunParamsDev rp, int slot, int out_buf, int ntx, int nty,
             int L)
@@ -288,7 +278,7 @@ k_march3d64(GridDev g, StateDev in, StateDev out, StepCtl* ctl, RunParamsDev rp,
                     top[v] = sh.hzT[v][tid];
                     sh.hzT[v][tid] = Uz[1][v];
                 }
-                march3d_riemann<LIM, RS, KIND>(e, top, Uz[0], 2, G);
+                march_riemann<3, RS>(e, top, Uz[0], 2, G);
                 if (z > zb && is_out) {
                     const int r = z - 1;
                     const int64_t o = r * plane2 + (int64_t)row * in.pitch + col;
@@ -378,7 +368,7 @@ k_march3d64(GridDev g, StateDev in, StateDev out, StepCtl* ctl, RunParamsDev rp,
                 for (int v = 0; v < 5; ++v) {
                     q[v] = in.q[o + v * in.plane]; // ahead of the solve, which hides the load
                 }
-                march3d_riemann<LIM, RS, KIND>(e, uL, uR, 0, F);
+                march_riemann<3, RS>(e, uL, uR, 0, F);
                 const double dtv = 2 * dthv; // dt / dv: dt = 2 dth
 #pragma unroll
                 for (int v = 0; v < 5; ++v) {
@@ -405,7 +395,7 @@ k_march3d64(GridDev g, StateDev in, StateDev out, StepCtl* ctl, RunParamsDev rp,
                 dn[v] = sh.face[3][v][tid - 32];
                 up[v] = sh.face[2][v][tid];
             }
-            march3d_riemann<LIM, RS, KIND>(e, dn, up, 1, G);
+            march_riemann<3, RS>(e, dn, up, 1, G);
 #pragma unroll
             for (int v = 0; v < 5; ++v) {
                 sh.face[2][v][tid] = G[v];

@@ -363,7 +363,6 @@ k_hydro_reconstruction(GridDev g, Box bx, double dt, const double* __restrict__ 
 // of 32 faces of one dimension; the tile's last x-faces form one more row.
 template <int ND>
 struct GodTile {
-    static constexpr int NV = ND + 2;
     static constexpr int T[3] = {ND == 1 ? kThreads : 32, ND == 1 ? 1 : (ND == 2 ? 8 : 4), ND == 3 ? 2 : 1};
     static constexpr int NF(int d)
     {
