@@ -2792,9 +2792,10 @@ int hcl_ensemble_adjoint(hcl_ensemble* e, const double* const* lam_final, double
 // ---- hydro reconstruction for callers whose loop must not allocate -----------------
 namespace {
 
-// The entry point's documented size limit: the scratch of the reference's
-// MUSCLHancockHydroReconstruction (u_rec, P_rec, fx_rec_old) in 32 MiB.
-constexpr size_t kNoAllocScratchDoubles = size_t(1) << 22;
+// The entry point's documented size limit, in the units of the reference's
+// MUSCLHancockHydroReconstruction scratch (u_rec, P_rec, fx_rec_old).  The one
+// kernel needs no scratch; callers rely on the limit's error.
+constexpr size_t kNoAllocLimitDoubles = size_t(1) << 22;
 
 } // namespace
 
@@ -2818,11 +2819,11 @@ int hcl_hydro_reconstruction_noalloc(hcl_handle* h, int ng_eff, double dt, const
     const size_t nd = (size_t)h->g.ndim;
     const size_t N = (size_t)h->g.N;
     const size_t n_u = N * 2 * nd * nd, n_p = N * 2 * nd, n_fx = N * 2 * nd * (size_t)h->g.nfx;
-    if (n_u + n_p + n_fx > kNoAllocScratchDoubles) {
+    if (n_u + n_p + n_fx > kNoAllocLimitDoubles) {
         return fail(HCL_ERR_CONFIG,
-                    "hcl_hydro_reconstruction_noalloc: this grid needs %zu scratch doubles (%zu cells x 2*ndim*(ndim+1+nfx)), "
-                    "the fixed buffer holds %zu; use hcl_hydro_reconstruction",
-                    n_u + n_p + n_fx, N, kNoAllocScratchDoubles);
+                    "hcl_hydro_reconstruction_noalloc: %zu doubles (%zu cells x 2*ndim*(ndim+1+nfx)) are more than the "
+                    "entry point's limit of %zu (its former fixed buffer); use hcl_hydro_reconstruction",
+                    n_u + n_p + n_fx, N, kNoAllocLimitDoubles);
     }
     int prev = -1;
     HCL_CUDA(cudaGetDevice(&prev));

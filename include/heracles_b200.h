@@ -172,9 +172,9 @@ int hcl_hydro_reconstruction(hcl_handle* h, int ng_eff, double dt, const double*
  * (its MUSCLHancockHydroReconstruction owns Kokkos views allocated at
  * construction).  Switches to the handle's device for the call.
  * Limit: N * 2*ndim*(ndim + 1 + nfx) <= 2^22 doubles, N the cell count with
- * ghosts (2-D, nfx = 0: N <= 349525; 3-D: N <= 174762), the size of the
- * scratch of the reference's separate kernels; larger grids get
- * HCL_ERR_CONFIG. */
+ * ghosts (2-D, nfx = 0: N <= 349525; 3-D: N <= 174762), the size that the
+ * scratch of the reference's separate kernels would have; the call itself
+ * needs none.  Larger grids get HCL_ERR_CONFIG. */
 int hcl_hydro_reconstruction_noalloc(hcl_handle* h, int ng_eff, double dt, const double* rho, const double* u,
                                      const double* P, const double* fx, double* rho_rec, double* rhou_rec,
                                      double* E_rec, double* fx_rec, void* stream);

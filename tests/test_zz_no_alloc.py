@@ -1,8 +1,8 @@
-"""hcl_hydro_reconstruction_noalloc (fixed device scratch, no allocation in
-the call) against hcl_hydro_reconstruction (the handle's own scratch), through
-the C ABI: identical face states on two calls in a row, and a clear error for
-grids whose scratch does not fit the fixed array.  Collected last so that it
-also runs after every other test of the session."""
+"""hcl_hydro_reconstruction_noalloc (no allocation in the call) through the C
+ABI: the same face states as hcl_hydro_reconstruction on two calls in a row (both
+run one kernel) and as the oracle, no device memory taken, and a clear error for
+grids beyond its documented limit.  Collected last so that it also runs after
+every other test of the session."""
 import ctypes as C
 
 import numpy as np
@@ -87,4 +87,36 @@ def test_noalloc_rejects_grids_beyond_the_fixed_scratch():
     assert rc != 0
     with pytest.raises(HclError, match="fixed buffer"):
         check(rc)
+    dom.close()
+
+
+@pytest.mark.parametrize("geometry", ["Cartesian", "Spherical"])
+@pytest.mark.parametrize("ndim,nx,nfx", [(1, [200], 1), (2, [64, 48], 0), (3, [20, 12, 16], 2)])
+def test_noalloc_matches_oracle_and_takes_no_memory(ndim, nx, nfx, geometry):
+    import torch
+
+    from heraclespp_b200 import Domain
+    from heraclespp_b200._native import check
+    from oracle import Oracle
+
+    L = noalloc_lib()
+    kw = dict(gamma=1.4, limiter="VanAlbada", riemann="HLL", g=(0.1, -0.2, 0.05), xmin=(0.4, 0.6, 0.1), xmax=(1.4, 2.2, 1.3))
+    dom = Domain(ndim, nx, nfx=nfx, geometry=geometry, **kw)
+    o = Oracle(ndim, nx, nfx=nfx, geom=geometry, **kw)
+    p = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+    fxp = lambda t: p(t) if nfx else None  # noqa: E731
+    rho, vel, P, fx = inputs(torch, dom, nfx, 5)
+    got = [torch.zeros_like(a) for a in outputs(torch, dom, nfx)]
+    host = lambda t, lead: t.cpu().numpy().reshape(lead + o.shape3)  # noqa: E731
+    ref = o.hydro_reconstruction(1, 2e-3, host(rho, ()), host(vel, (ndim,)), host(P, ()),
+                                 host(fx, (max(nfx, 1),)) if nfx else None)
+    free = []
+    for _ in range(2):  # the first call loads the kernel
+        check(L.hcl_hydro_reconstruction_noalloc(dom.h, 1, 2e-3, p(rho), p(vel), p(P), fxp(fx), p(got[0]), p(got[1]),
+                                                 p(got[2]), fxp(got[3]), None))
+        torch.cuda.synchronize()
+        free.append(torch.cuda.mem_get_info()[0])
+    assert free[0] == free[1]
+    for a, b in zip(got[: 4 if nfx else 3], ref):
+        np.testing.assert_array_equal(a.cpu().numpy().reshape(-1), b.reshape(-1))
     dom.close()
