@@ -55,3 +55,57 @@ def test_radgas(nx, nfx, lim, rs):
     assert np.allclose(log, dts, rtol=1e-12, atol=0)
     for a, ref in pairs:
         assert rel_l1(a, ref) < 1e-12
+
+
+# name: (grid arguments, nfx, pressure fix); 250 x 200 is 208 tiles of 16 x 16 and
+# 300 x 280 is 342: one partial and more than one wave at two CTAs per SM
+PERFECT = {
+    "cartesian": (dict(g=(0.03, -0.05, 0.0)), 0, False),
+    "spherical": (WEDGE, 0, False),
+    "point mass": (dict(gravity="Point_mass", central_mass=1e8, **WEDGE), 0, False),
+    "two scalars": (dict(), 2, False),
+    "spherical scalar": (WEDGE, 1, False),
+    "pressure fix": (dict(), 0, True),
+}
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp64_fast"])
+@pytest.mark.parametrize("lim,rs", [("VanLeer", "HLLC"), ("Minmod", "HLL"), ("VanAlbada", "Low Mach")])
+@pytest.mark.parametrize("name", PERFECT)
+@pytest.mark.parametrize("nx", [[250, 200], [300, 280]])
+def test_perfect_gas(nx, name, lim, rs, precision):
+    extra, nfx, fix = PERFECT[name]
+    kw = dict(gamma=1.4, limiter=lim, riemann=rs, bc=BC, **extra)
+    log, dts, pairs = run_both(nx, kw, nfx, pressure_fix=fix, precision=precision)
+    assert precision == "fp64_fast" or np.array_equal(log, dts)
+    for a, ref in pairs:
+        if precision == "fp64":
+            assert np.array_equal(a, ref)
+        else:
+            assert rel_l1(a, ref) < 1e-12  # the bound of the fast FP64 tests
+
+
+def stretched(nx, hi, ng=2):
+    """Widths that vary smoothly by a factor of two; the ghost widths repeat the
+    interior's."""
+    nodes = []
+    for n, h in zip(nx, hi):
+        s = (np.arange(n + 2 * ng + 1) - ng) / n
+        nodes.append(h * (s + 0.35 * np.sin(2 * np.pi * s) / (2 * np.pi)))
+    return nodes + [np.array([0.0, 1.0])] * (3 - len(nx))
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp64_fast"])
+@pytest.mark.parametrize("lim,rs", [("VanLeer", "HLLC"), ("Minmod", "HLL"), ("VanAlbada", "Low Mach"), ("Constant", "HLLC")])
+@pytest.mark.parametrize("nx", [[300, 280], [253, 310], [3, 4800]])
+def test_march_on_user_defined_nodes(nx, lim, rs, precision):
+    """The march divides by each column's and row's own widths."""
+    kw = dict(gamma=1.4, limiter=lim, riemann=rs, bc=["NullGradient", "Reflexive", "Periodic", "Periodic"],
+              nodes=stretched(nx, (1.0, 0.7)), xmax=(1.0, 0.7, 1.0), g=(0.03, -0.05, 0.0))
+    log, dts, pairs = run_both(nx, kw, precision=precision)
+    assert precision == "fp64_fast" or np.array_equal(log, dts)
+    for a, ref in pairs:
+        if precision == "fp64":
+            assert np.array_equal(a, ref)
+        else:
+            assert rel_l1(a, ref) < 1e-12
