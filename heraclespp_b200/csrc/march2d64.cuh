@@ -110,7 +110,7 @@ __device__ __forceinline__ q64::Den face_width(bool unif, double dl, double dl_p
         return q64::Den{1.0, 1.0};
     }
     const double h = (dl + dl_p) / 2;
-    return FAST ? q64::Den{h, 1.0 / h} : q64::den_any(h);
+    return FAST ? q64::Den{h, 1.0 / h} : q64::den(h);
 }
 
 template <int ND, int RS>

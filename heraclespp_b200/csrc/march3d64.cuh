@@ -105,7 +105,7 @@ k_march3d64(GridDev g, StateDev in, StateDev out, StepCtl* ctl, RunParamsDev rp,
         const bool x = k < kM3PX;
         const int d = x ? 0 : 1;
         const int c = min((x ? i0 - 2 + k : j0 - 2 + k - kM3PX), g.n[d] - 2);
-        const q64::Den h = raw ? q64::Den{1.0, 1.0} : q64::den_any((g.dx[d][c] + g.dx[d][c + 1]) / 2);
+        const q64::Den h = raw ? q64::Den{1.0, 1.0} : q64::den((g.dx[d][c] + g.dx[d][c + 1]) / 2);
         (x ? sh.hx[k] : sh.hy[k - kM3PX]) = h;
     }
 
@@ -194,8 +194,8 @@ k_march3d64(GridDev g, StateDev in, StateDev out, StepCtl* ctl, RunParamsDev rp,
                     hL = sh.hy[w];
                     hR = sh.hy[w + 1];
                 } else {
-                    hL = raw ? q64::Den{1.0, 1.0} : q64::den_any((g.dx[2][z - 1] + dlz) / 2);
-                    hR = raw ? q64::Den{1.0, 1.0} : q64::den_any((dlz + g.dx[2][z + 1]) / 2);
+                    hL = raw ? q64::Den{1.0, 1.0} : q64::den((g.dx[2][z - 1] + dlz) / 2);
+                    hR = raw ? q64::Den{1.0, 1.0} : q64::den((dlz + g.dx[2][z + 1]) / 2);
                 }
                 if constexpr (LIM == LIM_CONSTANT) {
 #pragma unroll

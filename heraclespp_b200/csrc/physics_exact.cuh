@@ -383,7 +383,8 @@ using plain::ek_cons;
 // its operands in a range S: denominators, pressures, and numerators, which may
 // be zero or smaller.  Where it holds every quotient and root is the rounded
 // one.  Otherwise the group is done again out of line: with quo_tiny() for the
-// numerators (TINY) if those were the matter, else with plain operators.  Scalings by powers of two (the /2 of the kinetic
+// numerators (TINY; the reference's arithmetic only) if those were the matter, else
+// with plain operators.  Scalings by powers of two (the /2 of the kinetic
 // energy, the 4/2 and 2/2 of the limiters) are folded, which is exact in that
 // range.
 template <int ND>
@@ -427,10 +428,10 @@ __device__ __forceinline__ void prim_core(const Eos& e, const double* c, double*
         }
         evol = c[1 + ND] - 0.5 * mu;
         p[1 + ND] = e.gamma_m1 * evol;
-        S.add(c[0], p[1 + ND]);
+        S.pos(c[0], p[1 + ND]);
         return;
     }
-    r = q64::den_any(c[0]);
+    r = q64::den(c[0]);
     double norm = 0;
 #pragma unroll
     for (int d = 0; d < ND; ++d) {
@@ -441,7 +442,7 @@ __device__ __forceinline__ void prim_core(const Eos& e, const double* c, double*
     const double kb = c[0] * kKb;
     k = q64::den_from(kb, r.y * (1 / kKb));
     p[1 + ND] = q64::quo(kb * q64::quo(evol * e.mmw * kMp * e.gamma_m1, k), e.mk);
-    S.add(c[0], p[1 + ND]);
+    S.pos(c[0], p[1 + ND]);
     S.low(kb);
     S.num(c[1], c[ND >= 2 ? 2 : 1]);
     if constexpr (ND == 3) {
@@ -452,13 +453,16 @@ template <int ND, int KIND>
 static __device__ __noinline__ void to_prim_slow(Eos e, const double* c, double* p)
 {
     e.kind = KIND;
-    q64::Den r, k;
-    double evol;
-    q64::Range S(e.consts_ok);
-    prim_core<ND, true>(e, c, p, r, k, evol, S);
-    if (!S.dens_ok()) {
-        plain::to_prim<ND>(e, c, p);
+    if constexpr (KIND == EOS_PERFECT_GAS) {
+        q64::Den r, k;
+        double evol;
+        q64::Range S(e.consts_ok);
+        prim_core<ND, true>(e, c, p, r, k, evol, S);
+        if (S.dens_ok()) {
+            return;
+        }
     }
+    plain::to_prim<ND>(e, c, p);
 }
 template <int ND>
 __device__ __forceinline__ void to_prim(const Eos& e, const double* c, double* p)
@@ -506,8 +510,7 @@ __device__ __forceinline__ void cons_flux_core(const Eos& e, const double* p, in
         evol = p[1 + ND] * (1.0 / e.gamma_m1);
     } else {
         const double kb = p[0] * kKb;
-        S.add(p[0], p[1 + ND]);
-        S.low(kb);
+        S.pos(p[0], p[1 + ND]);
         evol = evol_core(e, p[1 + ND], q64::den(kb));
     }
     double norm = 0;
@@ -583,8 +586,10 @@ template <int ND, int KIND>
 static __device__ __noinline__ void state_prims_slow(Eos e, const double* q, double* out)
 {
     e.kind = KIND;
-    if (e.kind != EOS_RAD_GAS && state_core<ND, true>(e, q, out[0], out[1], out + 2)) {
-        return;
+    if constexpr (KIND == EOS_PERFECT_GAS) {
+        if (state_core<ND, true>(e, q, out[0], out[1], out + 2)) {
+            return;
+        }
     }
     out[0] = q[1 + ND] - plain::ek_cons<ND>(q);
     plain::to_prim<ND>(e, q, out + 2);
@@ -644,11 +649,10 @@ __device__ __forceinline__ double limited_core(double dR, double dL, q64::Range&
     }
     S.slope(use, dR, dL, b);
     S.low(dL);
-    S.low(b);
     return use ? s : 0.0;
 }
-// The same for quotients down to 2^-1000, tiny pairs scaled by a power of two
-// (the slope scales with them); good turns false beyond that.
+// The same for quotients down to 2^-1000 of one sign, tiny pairs scaled by a power
+// of two (the slope scales with them); good turns false beyond that.
 template <int LIM>
 __device__ __forceinline__ double limited_tiny(double dR, double dL, bool& good)
 {
@@ -657,16 +661,16 @@ __device__ __forceinline__ double limited_tiny(double dR, double dL, bool& good)
     const bool use = !(dL * dR <= 0);
     const double up = lo < 0x1p-700 ? 0x1p400 : 1.0;
     const double down = lo < 0x1p-700 ? 0x1p-400 : 1.0;
-    const double R = dR * up, L = dL * up;
-    const double ratio = q64::quo(R, q64::den_any(L));
+    const double R = fabs(dR) * up, L = fabs(dL) * up;
+    const double ratio = q64::quo(R, q64::den(L));
     const double b = limited_den<LIM>(ratio);
     const double num = LIM == LIM_MINMOD ? fmin(1., ratio) : (R + L) * ratio;
-    double s = q64::quo(num, q64::den_any(b));
+    double s = q64::quo(num, q64::den(b));
     if constexpr (LIM == LIM_MINMOD) {
         s = s * (L + R);
     }
     good = !use || (lo >= 0x1p-1000 && hi <= 0x1p200 && ratio >= 0x1p-1000 && ratio <= 0x1p400);
-    return use ? s * down : 0.0;
+    return use ? copysign(s * down, dL) : 0.0;
 }
 // the raw-difference forms of the fast kind
 template <int LIM>
@@ -762,7 +766,7 @@ __device__ __forceinline__ void faces_lim(int kind, bool uniform, const double* 
     if (kind == EOS_PERFECT_GAS_FAST && uniform) {
         faces_den<NV, LIM>(kind, m, c, p, q64::Den{1.0, 1.0}, q64::Den{1.0, 1.0}, 0.5, lo, hi);
     } else {
-        faces_den<NV, LIM>(kind, m, c, p, q64::den_any((dl_m + dl) / 2), q64::den_any((dl + dl_p) / 2), dl / 2, lo, hi);
+        faces_den<NV, LIM>(kind, m, c, p, q64::den((dl_m + dl) / 2), q64::den((dl + dl_p) / 2), dl / 2, lo, hi);
     }
 }
 template <int NV>
@@ -890,11 +894,14 @@ template <int ND, int RS, int KIND>
 static __device__ __noinline__ void riemann_slow(Eos e, const double* cL, const double* cR, int l, double* f)
 {
     e.kind = KIND;
-    q64::Range S(e.consts_ok);
-    riemann_core<ND, RS, true>(e, cL, cR, l, f, S);
-    if (!S.dens_ok()) {
-        plain::riemann<ND>(e, RS, cL, cR, l, f);
+    if constexpr (KIND == EOS_PERFECT_GAS) {
+        q64::Range S(e.consts_ok);
+        riemann_core<ND, RS, true>(e, cL, cR, l, f, S);
+        if (S.dens_ok()) {
+            return;
+        }
     }
+    plain::riemann<ND>(e, RS, cL, cR, l, f);
 }
 template <int ND, int RS>
 __device__ __forceinline__ void riemann_rs(const Eos& e, const double* cL, const double* cR, int l, double* f)
