@@ -19,11 +19,12 @@ std::atomic<int64_t> g_launches{0};
 namespace {
 
 constexpr int kThreads = 256;
-// The two heaviest stage kernels (Hancock predictor, Godunov update) ask for
-// two CTAs per SM: three steps of 120 x 100 x 70 through the stage entry
-// points take 3.06 ms unbounded, 2.68 ms at two CTAs, 2.64 ms at three, which
-// spill 2.7 KB per thread; with a branch per division (three CTAs) 3.04 ms.
-constexpr int kHeavyMinBlocks = 2;
+// CTAs per SM that the two heaviest stage kernels are held to (120 x 100 x 70 cells,
+// Van Leer and HLLC): the reconstruction 161 us at two and 260 at three, where it
+// spills; the Godunov update 134 and 114 us (RadGas, waiting on branching
+// divisions: 2.02 and 1.77 ms).
+constexpr int kReconMinBlocks = 2;
+constexpr int kGodunovMinBlocks = 3;
 
 struct Box {
     int b[3];
@@ -173,7 +174,7 @@ __global__ void k_face_recon(GridDev g, Box bx, const double* __restrict__ var, 
 // at the copy rate).  The face states of all but the last dimension wait for
 // the increments of the others in shared memory, where registers would spill.
 template <int ND>
-__global__ void __launch_bounds__(kThreads, kHeavyMinBlocks)
+__global__ void __launch_bounds__(kThreads, kReconMinBlocks)
 k_hydro_reconstruction(GridDev g, Box bx, double dt, const double* __restrict__ rho, const double* __restrict__ u,
                        const double* __restrict__ P, const double* __restrict__ fx, double* __restrict__ rho_rec,
                        double* __restrict__ rhou_rec, double* __restrict__ E_rec, double* __restrict__ fx_rec,
@@ -376,7 +377,7 @@ struct GodTile {
 };
 
 template <int ND>
-__global__ void __launch_bounds__(kThreads, kHeavyMinBlocks) k_godunov(GridDev g, Box bx, double dt, const double* __restrict__ rho, const double* __restrict__ rhou,
+__global__ void __launch_bounds__(kThreads, kGodunovMinBlocks) k_godunov(GridDev g, Box bx, double dt, const double* __restrict__ rho, const double* __restrict__ rhou,
                           const double* __restrict__ E, const double* __restrict__ fx,
                           const double* __restrict__ rho_rec, const double* __restrict__ rhou_rec,
                           const double* __restrict__ E_rec, const double* __restrict__ fx_rec,
