@@ -358,7 +358,7 @@ __device__ __forceinline__ void store_images_3d(double* __restrict__ q, int64_t 
 // more resident CTAs fill those waits.  Where the shared memory of a launch
 // leaves room for them the 2-D FP64 tile runs two CTAs per SM (128 registers,
 // some spilled; KH 2048^2 with a passive scalar 1.75 ms per step unbounded,
-// 0.99 ms so).  The straight-line quotients hold more values at once than the
+// 0.98 ms so).  The straight-line quotients hold more values at once than the
 // branching divisions did: three CTAs (80 registers) spill 1.5 KB per thread.
 // RadGas still divides with a branch and waits more: three CTAs (1024^2, Minmod
 // and HLLC: 2.20 ms per step, two CTAs 2.69; 256^2, two tiles per SM, 213 and 202

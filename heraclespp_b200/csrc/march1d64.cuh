@@ -13,8 +13,8 @@
 // primitives ~1000, exchange and cluster barrier ~2000.
 //
 // us per step, FP64 / fast FP64, one kernel per step against this: 1024 cells
-// 7.6 / 6.9 -> 3.7 / 3.1, 4096 cells 7.8 / 6.9 -> 4.7 / 3.7, 8192 cells 8.1 /
-// 6.9 -> 6.8 / 4.9 (one SM's FP64 pipe takes over: 512 cells per CTA), which is
+// 7.6 / 6.9 -> 3.2 / 3.0, 4096 cells 7.8 / 6.9 -> 4.1 / 3.5, 8192 cells 8.1 /
+// 6.9 -> 6.0 / 4.9 (one SM's FP64 pipe takes over: 512 cells per CTA), which is
 // why the line lies there.
 //
 // The arithmetic per cell is the tile kernel's (KIND EOS_PERFECT_GAS: the

@@ -13,7 +13,7 @@
 // What bounds it: FP64 (a warp instruction every two cycles per scheduler; 1140
 // operations per cell with the halo lanes in the exact form: 0.26 ms for
 // 2048^2 at the full rate).  KH 2048^2: 1.02 (tile kernel, a branch per
-// division) -> 0.56 ms per step, FP64 pipe 57 % and issue slots 54 % busy, the
+// division) -> 0.51 ms per step, FP64 pipe 57 % and issue slots 55 % busy, the
 // rest waits on dependency chains; the register window (partial update, lower
 // flux, top face, row quotients, primitives: 20 doubles) and the straight-line
 // groups leave room for three warps per scheduler (one CTA of 12 warps per SM,

@@ -20,10 +20,11 @@
 // shared planes cannot hold (1.75 against 1.42 ms below; 16 warps of 128
 // registers).  Three barriers per plane order the planes.
 //
-// What bounds it: FP64 (45 % of the pipe with 42 % of the issue slots; three
+// What bounds it: FP64 (48 % of the pipe with 45 % of the issue slots; three
 // warps per scheduler wait on dependency chains and at the barriers).  A
 // 128^2 x 256 step, HLL and Minmod: 4.2 (8x8x4 tiles, a branch per division) ->
-// 2.2 (the same tiles with quot64.cuh) -> 1.42 ms.
+// 2.2 (the same tiles with quot64.cuh) -> 1.30 ms (1.42 while the columns past the
+// domain's edge, which repeat its last one, asked for a second look each).
 #pragma once
 
 #include <cuda_runtime.h>

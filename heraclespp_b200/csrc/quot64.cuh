@@ -8,7 +8,7 @@
 // residual correction (quo), all of it straight-line code that the compiler
 // interleaves freely.  FP64 tile kernels, a branch per division against these:
 // Sod 1024 cells 14.6 -> 7.6 us per step, 2-D KH 2048^2 with a passive scalar
-// 1.51 -> 1.10 ms, 3-D 128^2 x 256 with a passive scalar 5.2 -> 3.2 ms, all
+// 1.51 -> 0.98 ms, 3-D 128^2 x 256 with a passive scalar 5.2 -> 3.2 ms, all
 // with the same bits.
 //
 // Method: Newton's iteration on the hardware's reciprocal approximation, then
